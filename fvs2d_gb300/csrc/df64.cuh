@@ -31,6 +31,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 namespace fvs {
 
 struct df64 {
@@ -53,9 +55,9 @@ __host__ __device__ __forceinline__ df64 two_sum(float a, float b) {
   const float bp = s - a;
   return df64(s, (a - (s - bp)) + (b - bp));
 }
-__device__ __forceinline__ df64 two_prod(float a, float b) {
+__host__ __device__ __forceinline__ df64 two_prod(float a, float b) {
   const float p = a * b;
-  return df64(p, __fmaf_rn(a, b, -p));
+  return df64(p, fmaf(a, b, -p));
 }
 
 __device__ __forceinline__ df64 operator+(df64 x, df64 y) {
@@ -66,10 +68,11 @@ __device__ __forceinline__ df64 operator+(df64 x, df64 y) {
 }
 __device__ __forceinline__ df64 operator-(df64 x) { return df64(-x.hi, -x.lo); }
 __device__ __forceinline__ df64 operator-(df64 x, df64 y) { return x + (-y); }
-__device__ __forceinline__ df64 operator*(df64 x, df64 y) {
+// (host and device round alike: the layout folds coefficients with it)
+__host__ __device__ __forceinline__ df64 operator*(df64 x, df64 y) {
   const df64 c = two_prod(x.hi, y.hi);
-  const float t = __fmaf_rn(x.hi, y.lo, x.lo * y.lo);
-  const float cl = c.lo + __fmaf_rn(x.lo, y.hi, t);
+  const float t = fmaf(x.hi, y.lo, x.lo * y.lo);
+  const float cl = c.lo + fmaf(x.lo, y.hi, t);
   return fast_two_sum(c.hi, cl);
 }
 __device__ __forceinline__ df64 mul_fp(df64 x, float y) {

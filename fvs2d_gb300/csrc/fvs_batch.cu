@@ -172,7 +172,7 @@ int build_batch_device(fvs_batch* B, DevView& d) {
   B->nc = L.nc;
   B->ne = L.ne;
   B->ref_off = B->coff;  // L.perm is appended case by case in the same order
-  if (!upload_layout(B->arena, L, d)) return B->fail(FVS_ERR_NOMEM, "device allocation or upload of the batch meshes failed");
+  if (!upload_layout(B->arena, L, d, false, !fold_w)) return B->fail(FVS_ERR_NOMEM, "device allocation or upload of the batch meshes failed");
   if (first && !B->arena.upload(B->d_perm, L.perm)) return B->fail(FVS_ERR_NOMEM, "upload of the cell maps failed");
   double* dp = nullptr;
   if (!B->arena.upload(dp, B->pinf)) return B->fail(FVS_ERR_NOMEM, "upload of the free streams failed");

@@ -335,10 +335,10 @@ int build_device(fvs_handle* H) {
   H->perm = L.perm;
   DevView& d = H->d;
   int* dperm = nullptr;
-  if (!upload_layout(H->arena, L, d) || !H->arena.upload(dperm, L.perm))
+  if (!upload_layout(H->arena, L, d, fuse != 0, !fold_w) || !H->arena.upload(dperm, L.perm))
     return H->fail(FVS_ERR_NOMEM, "device allocation or upload of the mesh failed");
   H->d_perm = dperm;
-  H->nblk = (L.nc + 255) / 256;
+  H->nblk = (L.nc + 127) / 128;  // the update's shortest block
   void* p;
   if (!alloc_work<T>(H->arena, d, L.nc, L.ne, H->nblk, 4096) || !H->arena.alloc(p, 32 * (size_t)L.nc))
     return H->fail(FVS_ERR_NOMEM, "device allocation of the state failed");
@@ -389,7 +389,7 @@ void set_stages(fvs_handle* H) {
 void enqueue_step(fvs_handle* H) {
   const KernelSet& K = *H->ks;
   cudaStream_t s = H->stream;
-  K.begin_step(H->d, s);
+  if (H->tile_mode) K.begin_step(H->d, s);
   if (H->tile_mode == 1) {
     const DevView dv = H->tile_view();
     for (size_t k = 0; k < H->stages.size(); k++) K.tile_stage(dv, H->tv, H->stages[k], (int)k, s);
@@ -417,11 +417,11 @@ void enqueue_step(fvs_handle* H) {
 }
 
 int count_launches(const fvs_handle* H) {
-  // k_begin_step, then gradient (second order), flux and update per stage,
-  // or one fused tile stage; the last stage also reduces the norms
+  // gradient (second order), flux and update per stage, or k_begin_step and
+  // one fused tile stage; the last stage also reduces the norms
   const int grad = H->d.first_order ? 0 : 1;
   int per_stage = (H->tile_mode == 1 || H->tile_mode == 3) ? 1 : H->tile_mode == 2 ? grad + 1 : grad + 2;
-  return 1 + per_stage * (int)H->stages.size();
+  return (H->tile_mode ? 1 : 0) + per_stage * (int)H->stages.size();
 }
 
 int ensure_graph(fvs_handle* H, int steps_per_graph) {
@@ -463,8 +463,11 @@ int bounds_report(fvs_handle* H) {
 // residual of the current device state at `time` (stage-free): fills d.resid, d.ws
 int device_residual(fvs_handle* H, double time) {
   NvtxRange nv("fvs residual (gradient, flux, gather)");
+  // the flux kernel's time: tctl[0] at step 0
   H->h_small[0] = time;
-  cudaError_t e = cudaMemcpyAsync(H->d.tctl + 1, H->h_small, sizeof(double), cudaMemcpyHostToDevice, H->stream);
+  reinterpret_cast<int*>(H->h_small + 1)[0] = 0;
+  cudaError_t e = cudaMemcpyAsync(H->d.tctl, H->h_small, sizeof(double), cudaMemcpyHostToDevice, H->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(H->d.stepctl, H->h_small + 1, sizeof(int), cudaMemcpyHostToDevice, H->stream);
   if (e != cudaSuccess) return H->cuda_fail(e, "time upload");
   H->ks->cvar2pvar(H->d, H->stream);
   H->ks->gradient(H->d, H->stream);
@@ -1007,7 +1010,7 @@ int fvs_profile_step(fvs_handle* h, int32_t cap, int32_t* n, char* names, float*
   };
   if ((rc = refill_gather(h))) return rc;
   mark("start");
-  K.begin_step(h->d, s);
+  if (h->tile_mode) K.begin_step(h->d, s);
   if (h->tile_mode == 1) {
     const DevView dv = h->tile_view();
     for (size_t k = 0; k < h->stages.size(); k++) {

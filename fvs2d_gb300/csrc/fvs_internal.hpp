@@ -107,13 +107,19 @@ struct DevView {
   const int4* cflist = nullptr;  // [nc] signed flux slots, reference summation order
   const void* cpos = nullptr;    // [nc][4] x 2 face-centre offsets (T) for the limiter
   const int8_t* nvrt = nullptr;
+  // gradient stencil interleaved over groups of 32 cells: entry j of cell ic
+  // at ell_base[ic / 32] + 32 j + ic % 32, j < ell_n[ic]
+  const int* ell_base = nullptr;
+  const uint8_t* ell_n = nullptr;
+  const int* ell_cell = nullptr;
+  const void* ell_coef = nullptr;  // x 2 (T); GGNB: edge times node coefficient
+  const void* ell_w = nullptr;     // LSQ weights (T), strict build
+  const void* coef0 = nullptr;     // [nc] x 2 (T)
+  // the same stencil as CSR rows (fused tile stages only)
   const int* st_ptr = nullptr;
-  const int* st_cell = nullptr;
-  const void* st_coef = nullptr;  // LSQ/GGCB [len] x 2 (T); GGNB [len] (T)
-  const void* st_w = nullptr;     // LSQ [len] (T)
+  const void* st_coef = nullptr;   // LSQ/GGCB [len] x 2 (T); GGNB [len] (T)
   const int8_t* st_node = nullptr;
-  const void* coef0 = nullptr;    // [nc] x 2 (T)
-  const void* coefedg = nullptr;  // [nc][4] x 2 (T)
+  const void* coefedg = nullptr;   // [nc][4] x 2 (T)
   // edges
   const int2* ecell = nullptr;    // (L,R) device cell ids; R = -1 on boundary edges
   const void* enrm = nullptr;     // [nedge] x 2 unit normal (T)
@@ -131,9 +137,10 @@ struct DevView {
   int norm_cap = 0;
   int* bounds_err = nullptr;      // [4] index-checking kernels: flag, site, index, extent
   int* stepctl = nullptr;         // [0] = steps done in this call
+  int trig_first = 0;             // the launch's pdl_trigger before its work (else after it)
   int upd_grid = 0;               // blocks of the last stage's update launch, which strides over the cells
                                   // (one wave of resident blocks; 0: one block per 256 cells)
-  double* tctl = nullptr;         // [0] = t1, [1] = told of the current step
+  double* tctl = nullptr;         // [0] = t1 of the call, [1] = time of the current step (tile stages)
   // scheme
   double gamma = 1.4, khalf = 0, nkhalf = 0, omk = 1, cfl = 1, dt = 0;
   double gm1 = 0.4, igm1 = 2.5, ggm1 = 3.5;  // gamma-1, 1/(gamma-1) and gamma/(gamma-1)
@@ -277,7 +284,7 @@ struct PersistPlan {
 // FMA, mixed).  All launch on the given stream; none synchronises.
 struct KernelSet {
   const char* name;
-  void (*begin_step)(const DevView&, cudaStream_t);
+  void (*begin_step)(const DevView&, cudaStream_t);  // tile stages: tctl[1]
   void (*cvar2pvar)(const DevView&, cudaStream_t);
   void (*gradient)(const DevView&, cudaStream_t);
   // ws_out: also store the wave-speed records (a steady scheme's first stage

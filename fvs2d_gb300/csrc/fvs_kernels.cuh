@@ -77,11 +77,27 @@ __device__ __forceinline__ int chk_idx(int* err, int i, int lo, int hi, int site
 // a kernel's blocks may be scheduled while its predecessor in the stream
 // finishes.  pdl_wait() blocks until the predecessor grid has completed and
 // its memory writes are visible; every kernel calls it before its first
-// global memory access, so results are unchanged.  pdl_trigger() right after
-// lets this grid's successor be launched once every block of this grid has
-// started.  Launched without the attribute, both return at once.
+// access to anything that a kernel of a step writes (the mesh arrays, fixed
+// since the handle was built, are read ahead of it).  pdl_trigger() lets this
+// grid's successor be launched once every block of this grid has reached it.
+// Called before the work, the successor's blocks are placed while this grid
+// runs and its mesh loads overlap with it, but they go to the SMs that have
+// room left, unevenly: a grid of less than a few waves then runs twice over on
+// some SMs.  So the step kernels call it before their work where the grid
+// leaves half of the 152 SMs free (SSP-RK3 step, before / after the work:
+// double-float 2,048 cells 34.8 / 45.1 us, 8,192 cells 42.9 / 44.9) and where it fills the chip for
+// several waves (mixed 524,000 cells 104.8 / 108.5 us, FP64 264,000 cells 449 / 458), and after it in between
+// (FP64 8,192 cells 89.5 / 49.1 us, 32,000 cells 155 / 84, 131,000 cells 262 /
+// 248; mixed 131,000 cells 44.9 / 38.9).  Launched without the attribute, both return at once.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// time at the start of the current step, told = t1 + (istep-1)*dt
+// (src/runge_kutta.f90:207-208), from t1 and the steps done, both on the
+// device (a captured step replays with its own time).  The flux kernel reads
+// it on boundary slots only; the fused tile stages read it from tctl[1],
+// where their k_begin_step puts it.
+__device__ __forceinline__ double told_of(const DevView& d) { return d.tctl[0] + double(d.stepctl[0]) * d.dt; }
 
 // programmatic dependent launch of the single-mesh step kernels (see
 // pdl_wait); FVS2D_PDL=0 in the environment launches them plainly
@@ -92,6 +108,25 @@ static bool pdl_enabled() {
   }();
   return on;
 }
+
+// Threads per block of the gradient, flux and update launches (items are
+// independent, one per thread).  The FP64 kernels keep an SM's FP64 pipe (2
+// operations per clock) busy with a few warps, so what counts is that every SM
+// gets the same number of warps: short blocks even that out where the mesh
+// is a few waves or less (SSP-RK3 step, blocks of 256 / 128 / 64: 8,192 cells
+// 71 / 51 / 51 us, 32,000 cells 102 / 88 / 90, 131,000 cells 268 / 248 / 258;
+// 65,024 limited quadrilaterals with 8-entry stencils 636 / 616 / 563;
+// 524,000 cells 875 / 857 / 858).  The update ends in a block reduction at the
+// last stage and keeps longer blocks.  Double-float lies in between (8,192
+// cells 48.6 / 46.9 / 47.3 us, 131,000 cells 92.6 / 88.9 / 98.4); mixed waits on memory
+// and wants the fewest blocks (131,000 cells 41.1 / 43.1 / 59.6 us).
+#if FVS_MIXED
+constexpr unsigned BLK_GRADIENT = 256, BLK_FLUX = 256, BLK_UPDATE = 256;
+#elif FVS_DF
+constexpr unsigned BLK_GRADIENT = 128, BLK_FLUX = 128, BLK_UPDATE = 128;
+#else
+constexpr unsigned BLK_GRADIENT = 64, BLK_FLUX = 64, BLK_UPDATE = 128;
+#endif
 
 template <typename... KArgs, typename... Args>
 static void launch_k(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
@@ -224,6 +259,30 @@ __device__ __forceinline__ float dabs_(float x) { return fabsf(x); }
 __device__ __forceinline__ double half(double x) { return 0.5 * x; }
 __device__ __forceinline__ float half(float x) { return 0.5f * x; }
 
+// a < b, and the sign of a number, without the FP64 pipe: FP64 compares issue
+// there, 2 per clock and SM; the bit patterns of ordered numbers compare as
+// integers once a negative pattern's magnitude is flipped.  For numbers that
+// are not NaN.
+#if FVS_FP64_FAST
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ bool less_than(double a, double b) { return order_key(a) < order_key(b); }
+// x > 0 and not NaN: the patterns 1 .. Inf
+__device__ __forceinline__ bool is_positive(double x) {
+  return (unsigned long long)(__double_as_longlong(x) - 1) < 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ bool is_negative(double x) { return is_positive(-x); }
+#else
+template <typename R>
+__device__ __forceinline__ bool less_than(R a, R b) { return a < b; }
+template <typename R>
+__device__ __forceinline__ bool is_positive(R x) { return x > R(0); }
+template <typename R>
+__device__ __forceinline__ bool is_negative(R x) { return x < R(0); }
+#endif
+
 #if FVS_MIXED
 // FP32 limiter with every product and sum pinned (explicit multiply-adds),
 // so that the compiler's contraction choices cannot differ between the
@@ -243,6 +302,22 @@ __device__ __forceinline__ float limiter_fn(int type, float a, float b, float ep
 // a face value p + cx gx + cy gy with the same pinned sequence
 __device__ __forceinline__ float face_value(float p, float cx, float gx, float cy, float gy) {
   return __fmaf_rn(cy, gy, __fmaf_rn(cx, gx, p));
+}
+#elif FVS_FP64_FAST
+// limiter, src/gradient_limiter.f90:103-134 (eps2 precomputed per cell), with
+// fused multiply-adds and the refined reciprocal (den > 0 for the
+// Venkatakrishnan form: a a + a b + 2 b b + eps2 with a, b of one sign)
+__device__ __forceinline__ double limiter_fn(int type, double a, double b, double eps2) {
+  if (type == FVS_LIM_VENK) {
+    const double q = fma(a, a, eps2);
+    return fma(2.0 * a, b, q) * rcp_nr(fma(b, fma(2.0, b, a), q));
+  }
+  if (type == FVS_LIM_BARTH) { const double q = a / b; return q < 1.0 ? q : 1.0; }
+  const double l = fma(fma(b, b, eps2), a, fma(a, a, eps2) * b) / fma(2.0, eps2, fma(a, a, b * b));
+  return l / (b + eps2);
+}
+__device__ __forceinline__ double face_value(double p, double cx, double gx, double cy, double gy) {
+  return fma(cy, gy, fma(cx, gx, p));
 }
 #else
 // limiter, src/gradient_limiter.f90:103-134 (eps2 precomputed per cell)
@@ -437,134 +512,175 @@ __device__ __forceinline__ void roe_flux_area_fp64(double gm1, double ggm1, cons
 // ---------------------------------------------------------------------------
 // gradient (+ limiter) : one thread per cell
 // ---------------------------------------------------------------------------
-// Gradient (and limiter) of cell ic from its primitives pc; load(k, pj)
-// fills pj with the primitives of stencil entry k (global CSR index).
-// Shared by the separate gradient kernel (loads from global memory) and the
-// fused tile stage (loads from shared memory): the same arithmetic.
-// gradient_core over the stencil entries [b, e) with coef(k) the (LSQ or
-// GG-cell) coefficient pair of entry k
-template <int METHOD, int LIM, class Load, class Coef>
-__device__ __forceinline__ void gradient_core_r(const DevView& d, int ic, const T* pc, int b, int e, Load load,
-                                                Coef coef, T* gx, T* gy, T& phi_out) {
-  T pmin[4], pmax[4];
+// Gradient sums of one cell over its stencil entries, and the running
+// extrema the limiter needs.  Shared by the separate gradient kernel
+// (entries from the interleaved stencil, gathers from global memory) and the
+// fused tile stages (entries from the CSR stencil, values from shared
+// memory): the same arithmetic in the same entry order.
+template <int METHOD, int LIM>
+struct GradSum {
+  T gx[4], gy[4], pmin[4], pmax[4];
+
+  // pc: the cell's primitives; c0: its own coefficient pair (Green-Gauss)
+  __device__ __forceinline__ void init(const T* pc, T2 c0) {
 #pragma unroll
-  for (int v = 0; v < 4; v++) { pmin[v] = pc[v]; pmax[v] = pc[v]; }
-  if (METHOD == FVS_GRAD_LSQ) {
-    // grad_lsq, src/gradient_lsq.f90:393-401: sum over the stencil of
-    // (coef * (p_j - p_i)) * w, stencil outer, variable inner
+    for (int v = 0; v < 4; v++) {
+      pmin[v] = pc[v];
+      pmax[v] = pc[v];
+      gx[v] = METHOD == FVS_GRAD_LSQ ? T(0) : c0.x * pc[v];
+      gy[v] = METHOD == FVS_GRAD_LSQ ? T(0) : c0.y * pc[v];
+    }
+  }
+
+  // one entry: neighbour values pj, coefficient pair c; w: the LSQ weight of
+  // the strict build (other builds fold it into c on the host)
+  __device__ __forceinline__ void add(const T* pc, const T* pj, T2 c, T w) {
 #pragma unroll
-    for (int v = 0; v < 4; v++) { gx[v] = T(0); gy[v] = T(0); }
-#if FVS_STRICT
-    const T* __restrict__ W = static_cast<const T*>(d.st_w);
-#endif
-    for (int k = b; k < e; k++) {
-      T pj[4];
-      load(k, pj);
-      const T2 c = coef(k);
-#if FVS_STRICT
-      const T w = W[k];
-#endif
-#pragma unroll
-      for (int v = 0; v < 4; v++) {
+    for (int v = 0; v < 4; v++) {
+      if (METHOD == FVS_GRAD_LSQ) {
+        // grad_lsq, src/gradient_lsq.f90:393-401: sum over the stencil of
+        // (coef * (p_j - p_i)) * w
         const T diff = pj[v] - pc[v];
 #if FVS_STRICT
         gx[v] = gx[v] + c.x * diff * w;
         gy[v] = gy[v] + c.y * diff * w;
 #elif FVS_DF
-        // coefficients premultiplied by the weight on the host
         gx[v] = dfma(c.x, diff, gx[v]);
         gy[v] = dfma(c.y, diff, gy[v]);
 #else
-        // coefficients premultiplied by the weight on the host
         gx[v] = gx[v] + c.x * diff;
         gy[v] = gy[v] + c.y * diff;
 #endif
-        if (LIM) {
-          pmin[v] = pj[v] < pmin[v] ? pj[v] : pmin[v];
-          pmax[v] = pj[v] > pmax[v] ? pj[v] : pmax[v];
-        }
-      }
-    }
-  } else if (METHOD == FVS_GRAD_GGCB) {
-    // grad_ggcb, src/gradient_ggcb.f90:123-135
-    const T2 c0 = ld2(d.coef0, ic);
-#pragma unroll
-    for (int v = 0; v < 4; v++) { gx[v] = c0.x * pc[v]; gy[v] = c0.y * pc[v]; }
-    for (int k = b; k < e; k++) {
-      T pj[4];
-      load(k, pj);
-      const T2 c = coef(k);
-#pragma unroll
-      for (int v = 0; v < 4; v++) {
+      } else {
+        // grad_ggcb, src/gradient_ggcb.f90:123-135; grad_ggnb,
+        // src/gradient_ggnb.f90:190-207 (c: edge times node coefficient)
 #if FVS_DF
-        gx[v] = dfma(c.x, pj[v], gx[v]);
-        gy[v] = dfma(c.y, pj[v], gy[v]);
-#else
+        if (METHOD == FVS_GRAD_GGCB) {
+          gx[v] = dfma(c.x, pj[v], gx[v]);
+          gy[v] = dfma(c.y, pj[v], gy[v]);
+          continue;
+        }
+#endif
         gx[v] = gx[v] + c.x * pj[v];
         gy[v] = gy[v] + c.y * pj[v];
-#endif
+      }
+      if (LIM) {
+        pmin[v] = less_than(pj[v], pmin[v]) ? pj[v] : pmin[v];
+        pmax[v] = less_than(pmax[v], pj[v]) ? pj[v] : pmax[v];
       }
     }
-#if FVS_STRICT
-    const T vol = d.vol[ic];
-#pragma unroll
-    for (int v = 0; v < 4; v++) { gx[v] = gx[v] / vol; gy[v] = gy[v] / vol; }
-#else
-    const T rv = static_cast<const T*>(d.volT)[ic];
-#pragma unroll
-    for (int v = 0; v < 4; v++) { gx[v] = gx[v] * rv; gy[v] = gy[v] * rv; }
-#endif
-  } else {
-    // grad_ggnb, src/gradient_ggnb.f90:190-207
-    const T2 c0 = ld2(d.coef0, ic);
-#pragma unroll
-    for (int v = 0; v < 4; v++) { gx[v] = c0.x * pc[v]; gy[v] = c0.y * pc[v]; }
-    const T* __restrict__ CN = static_cast<const T*>(d.st_coef);
-    for (int k = b; k < e; k++) {
-      T pj[4];
-      load(k, pj);
-      const T cn = CN[k];
-      const T2 ce = ld2(d.coefedg, 4 * ic + d.st_node[k]);
-#pragma unroll
-      for (int v = 0; v < 4; v++) { gx[v] = gx[v] + ce.x * cn * pj[v]; gy[v] = gy[v] + ce.y * cn * pj[v]; }
-    }
-#if FVS_STRICT
-    const T vol = d.vol[ic];
-#pragma unroll
-    for (int v = 0; v < 4; v++) { gx[v] = gx[v] / vol; gy[v] = gy[v] / vol; }
-#else
-    const T rv = static_cast<const T*>(d.volT)[ic];
-#pragma unroll
-    for (int v = 0; v < 4; v++) { gx[v] = gx[v] * rv; gy[v] = gy[v] * rv; }
-#endif
+    (void)w;
   }
-  if (LIM) {
-    // compute_gradient_limiter, src/gradient_limiter.f90:47-88
-    const int nv = d.nvrt[ic];
-    const T eps2 = static_cast<const T*>(d.eps2)[ic];
-    T2 cp[4];
+
+  // Green-Gauss: divide by the volume; limiter value
+  __device__ __forceinline__ void finish(const DevView& d, int ic, const T* pc, T& phi_out) {
+    if (METHOD != FVS_GRAD_LSQ) {
+#if FVS_STRICT
+      const T vol = d.vol[ic];
 #pragma unroll
-    for (int f = 0; f < 4; f++) cp[f] = ld2(d.cpos, 4 * ic + f);
-    T phimin = T(1);
+      for (int v = 0; v < 4; v++) { gx[v] = gx[v] / vol; gy[v] = gy[v] / vol; }
+#else
+      const T rv = static_cast<const T*>(d.volT)[ic];
 #pragma unroll
-    for (int v = 0; v < 4; v++) {
-      T pe[4] = {T(100), T(100), T(100), T(100)};
-#pragma unroll
-      for (int f = 0; f < 4; f++) {
-        if (f >= nv) break;
-        const T pf = face_value(pc[v], cp[f].x, gx[v], cp[f].y, gy[v]);
-        const T dmax = pmax[v] - pc[v], dmin = pmin[v] - pc[v], diff = pf - pc[v];
-        if (diff > T(0)) pe[f] = limiter_fn(d.limiter, dmax, diff, eps2);
-        else if (diff < T(0)) pe[f] = limiter_fn(d.limiter, dmin, diff, eps2);
-        else pe[f] = T(1);
-      }
-      T mv = pe[0];
-#pragma unroll
-      for (int f = 1; f < 4; f++) mv = pe[f] < mv ? pe[f] : mv;
-      const T ph = mv < T(1) ? mv : T(1);
-      phimin = (v == 0 || ph < phimin) ? ph : phimin;
+      for (int v = 0; v < 4; v++) { gx[v] = gx[v] * rv; gy[v] = gy[v] * rv; }
+#endif
     }
-    phi_out = phimin;
+    if (LIM) {
+      // compute_gradient_limiter, src/gradient_limiter.f90:47-88
+      const int nv = d.nvrt[ic];
+      const T eps2 = static_cast<const T*>(d.eps2)[ic];
+      T2 cp[4];
+#pragma unroll
+      for (int f = 0; f < 4; f++) cp[f] = ld2(d.cpos, 4 * ic + f);
+      T phimin = T(1);
+#if FVS_FP64_FAST || FVS_DF
+      if (d.limiter != FVS_LIM_ALBADA) {
+        // The Venkatakrishnan and Barth functions of (a, b), a the stencil's
+        // extreme difference and b the face's, fall with growing |b| wherever
+        // they are below 1 (Venkatakrishnan: only for |b| > |a| / 2, where
+        // its derivative has the sign of (a a + eps2)(a - 4 b) - 4 a b b < 0), so the smallest
+        // value over a cell's faces, capped at 1, is that of the largest face difference of
+        // either sign: two evaluations per variable instead of one per face.
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+          T up = T(0), dn = T(0);
+#pragma unroll
+          for (int f = 0; f < 4; f++) {
+            if (f >= nv) break;
+            const T diff = face_value(pc[v], cp[f].x, gx[v], cp[f].y, gy[v]) - pc[v];
+            if (is_positive(diff) && less_than(up, diff)) up = diff;
+            if (is_negative(diff) && less_than(diff, dn)) dn = diff;
+          }
+          if (is_positive(up)) {
+            const T l = limiter_fn(d.limiter, pmax[v] - pc[v], up, eps2);
+            phimin = less_than(l, phimin) ? l : phimin;
+          }
+          if (is_negative(dn)) {
+            const T l = limiter_fn(d.limiter, pmin[v] - pc[v], dn, eps2);
+            phimin = less_than(l, phimin) ? l : phimin;
+          }
+        }
+        phi_out = phimin;
+        return;
+      }
+#endif
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        T pe[4] = {T(100), T(100), T(100), T(100)};
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+          if (f >= nv) break;
+          const T pf = face_value(pc[v], cp[f].x, gx[v], cp[f].y, gy[v]);
+          const T dmax = pmax[v] - pc[v], dmin = pmin[v] - pc[v], diff = pf - pc[v];
+          if (diff > T(0)) pe[f] = limiter_fn(d.limiter, dmax, diff, eps2);
+          else if (diff < T(0)) pe[f] = limiter_fn(d.limiter, dmin, diff, eps2);
+          else pe[f] = T(1);
+        }
+        T mv = pe[0];
+#pragma unroll
+        for (int f = 1; f < 4; f++) mv = pe[f] < mv ? pe[f] : mv;
+        const T ph = mv < T(1) ? mv : T(1);
+        phimin = (v == 0 || ph < phimin) ? ph : phimin;
+      }
+      phi_out = phimin;
+    }
+  }
+};
+
+// own coefficient pair of a cell (Green-Gauss gradients)
+template <int METHOD>
+__device__ __forceinline__ T2 own_coef(const DevView& d, int ic) {
+  T2 c = {T(0), T(0)};
+  if (METHOD != FVS_GRAD_LSQ) c = ld2(d.coef0, ic);
+  return c;
+}
+
+#if FVS_MIXED || FVS_DF
+// The fused tile stages' form: stencil entries [b, e) of the CSR stencil,
+// load(k, pj) fills pj with the primitives of entry k, coef(k) its (LSQ or
+// GG-cell) coefficient pair.
+template <int METHOD, int LIM, class Load, class Coef>
+__device__ __forceinline__ void gradient_core_r(const DevView& d, int ic, const T* pc, int b, int e, Load load,
+                                                Coef coef, T* gx, T* gy, T& phi_out) {
+  GradSum<METHOD, LIM> s;
+  s.init(pc, own_coef<METHOD>(d, ic));
+  for (int k = b; k < e; k++) {
+    T pj[4];
+    load(k, pj);
+    if (METHOD == FVS_GRAD_GGNB) {
+      const T cn = static_cast<const T*>(d.st_coef)[k];
+      const T2 ce = ld2(d.coefedg, 4 * ic + d.st_node[k]);
+      const T2 c = {ce.x * cn, ce.y * cn};
+      s.add(pc, pj, c, T(1));
+    } else {
+      s.add(pc, pj, coef(k), T(1));
+    }
+  }
+  s.finish(d, ic, pc, phi_out);
+#pragma unroll
+  for (int v = 0; v < 4; v++) {
+    gx[v] = s.gx[v];
+    gy[v] = s.gy[v];
   }
 }
 
@@ -574,26 +690,113 @@ __device__ __forceinline__ void gradient_core(const DevView& d, int ic, const T*
   gradient_core_r<METHOD, LIM>(d, ic, pc, d.st_ptr[ic], d.st_ptr[ic + 1], load,
                                [&](int k) { return ld2(d.st_coef, k); }, gx, gy, phi_out);
 }
+#endif
 
+// Up to CH entries of a cell's stencil, loaded together so that their gathers
+// are in flight at the same time.  The stencil is interleaved over groups of
+// 32 consecutive cells (Layout::build_ell): entry j of the cells of a group
+// lies in 32 consecutive places, so a warp's loads of ids and coefficients are
+// contiguous.  (From CSR rows, 18 entries apart from cell to cell, and one
+// dependent gather at a time, the step of 524,288 cells with GG-node gradients
+// took 310 us in mixed precision, 180 us so.)
+template <int CH>
+struct StencilChunk {
+  int id[CH];
+  T2 c[CH];
+#if FVS_STRICT
+  T w[CH];
+#endif
+  // entries [j0, j0 + CH) below n; at: the cell's place of entry 0
+  __device__ __forceinline__ void load(const DevView& d, int at, int j0, int n) {
+#pragma unroll
+    for (int q = 0; q < CH; q++) {
+      const int k = at + 32 * (j0 + q);
+      if (j0 + q < n) {
+        id[q] = chk_idx(d.bounds_err, d.ell_cell[k], 0, d.nc, SITE_STENCIL);
+        c[q] = ld2(d.ell_coef, k);
+#if FVS_STRICT
+        w[q] = d.ell_w ? static_cast<const T*>(d.ell_w)[k] : T(1);
+#endif
+      }
+    }
+  }
+};
+
+// Gradient (and limiter) of one cell in two parts: the stencil's first
+// entries, which no kernel of a step writes, then everything that depends on
+// the primitives.
+template <int METHOD, int LIM, bool COH, int CH>
+struct GradientItem {
+  int at, n;
+  T2 c0;
+  StencilChunk<CH> ch;
+
+  __device__ __forceinline__ void load_static(const DevView& d, int ic) {
+    at = d.ell_base[ic >> 5] + (ic & 31);
+    n = d.ell_n[ic];
+    c0 = own_coef<METHOD>(d, ic);
+    ch.load(d, at, 0, n);
+  }
+  __device__ __forceinline__ void run(const DevView& d, int ic) {
+    const T* P = static_cast<const T*>(d.Pv);
+    T pc[4];
+    ldc4<COH>(P, ic, pc);
+    GradSum<METHOD, LIM> s;
+    s.init(pc, c0);
+    for (int j0 = 0;;) {
+      T pj[CH][4];
+#pragma unroll
+      for (int q = 0; q < CH; q++)
+        if (j0 + q < n) ldc4<COH>(P, ch.id[q], pj[q]);
+#pragma unroll
+      for (int q = 0; q < CH; q++)
+        if (j0 + q < n) {
+#if FVS_STRICT
+          s.add(pc, pj[q], ch.c[q], ch.w[q]);
+#else
+          s.add(pc, pj[q], ch.c[q], T(1));
+#endif
+        }
+      j0 += CH;
+      if (j0 >= n) break;
+      ch.load(d, at, j0, n);
+    }
+    T ph;
+    s.finish(d, ic, pc, ph);
+    st4(static_cast<T*>(d.Gx), ic, s.gx);
+    st4(static_cast<T*>(d.Gy), ic, s.gy);
+    if (LIM) static_cast<T*>(d.phi)[ic] = ph;
+  }
+};
+
+// (one entry at a time: the batch's kernels, whose register budget is set by
+// their flux)
 template <int METHOD, int LIM, bool COH>
 __device__ __forceinline__ void gradient_item(const DevView& d, int ic) {
-  const T* P = static_cast<const T*>(d.Pv);
-  T pc[4], gx[4], gy[4], ph;
-  ldc4<COH>(P, ic, pc);
-  gradient_core<METHOD, LIM>(
-      d, ic, pc, [&](int k, T* pj) { ldc4<COH>(P, chk_idx(d.bounds_err, d.st_cell[k], 0, d.nc, SITE_STENCIL), pj); },
-      gx, gy, ph);
-  st4(static_cast<T*>(d.Gx), ic, gx);
-  st4(static_cast<T*>(d.Gy), ic, gy);
-  if (LIM) static_cast<T*>(d.phi)[ic] = ph;
+  GradientItem<METHOD, LIM, COH, 1> g;
+  g.load_static(d, ic);
+  g.run(d, ic);
 }
 
+// Entries in flight per thread and blocks of 256 threads an SM must hold (a
+// bound on the registers) of the gradient kernel.  FP32: three entries, the
+// stencil of a triangle, at 48 registers (SSP-RK3 step of 1,048,576 cells: 191 us;
+// 2 entries at 40 registers 196, 3 unbounded 196, 4 at 64 registers 198; GG-node, 524,288
+// cells: 2 entries 196, 3 180).  Double-float: two entries at 64 registers (509 us;
+// 1 entry 513, 3 entries 528, 4 entries 535).  FP64 waits on its pipe, not on registers: 4
+// entries shorten the small meshes' chain (8,192 cells 47.6 us, 2 entries 49.1).
+constexpr int GRAD_CHUNK = FVS_MIXED ? 3 : FVS_DF ? 2 : 4;
+constexpr int grad_min_blocks(int lim) { return FVS_MIXED ? (lim ? 4 : 5) : FVS_DF ? (lim ? 2 : 4) : 1; }
+
 template <int METHOD, int LIM>
-__global__ void __launch_bounds__(256) k_gradient(const DevView d) {
-  pdl_wait();
-  pdl_trigger();
+__global__ void __launch_bounds__(256, grad_min_blocks(LIM)) k_gradient(const DevView d) {
   const int ic = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ic < d.nc) gradient_item<METHOD, LIM, false>(d, ic);
+  GradientItem<METHOD, LIM, false, GRAD_CHUNK> g;
+  if (ic < d.nc) g.load_static(d, ic);
+  pdl_wait();
+  if (d.trig_first) pdl_trigger();
+  if (ic < d.nc) g.run(d, ic);
+  if (!d.trig_first) pdl_trigger();
 }
 
 // ---------------------------------------------------------------------------
@@ -763,8 +966,9 @@ __device__ __forceinline__ void flux_finish(const DevView& d, int e, const T* pf
 // interior slot, its R cell; a boundary slot's right state is the ghost
 // state.  REC_FIRST reads no gradient; REC_SPEC no limiter value.  Shared by
 // the edge-flux kernel and the fused tile stage: the same arithmetic.
-template <int REC>
-__device__ __forceinline__ void face_states(const DevView& d, int e, bool interior, double time, T2 n, T2 dl, T2 dr,
+// time(): the stage's time, evaluated on boundary slots only.
+template <int REC, class Time>
+__device__ __forceinline__ void face_states(const DevView& d, int e, bool interior, Time time, T2 n, T2 dl, T2 dr,
                                             const T* pl, const T* gxl, const T* gyl, T phiL, const T* pr,
                                             const T* gxr, const T* gyr, T phiR, T* pfL, T* pfR) {
   constexpr bool SPEC = REC == REC_SPEC;
@@ -776,7 +980,7 @@ __device__ __forceinline__ void face_states(const DevView& d, int e, bool interi
       for (int v = 0; v < 4; v++) pfR[v] = pr[v];
     } else {
       const T2 xy = ld2(d.exy, e);
-      ghost_state(d, d.ebtype[e], time, xy.x, xy.y, n.x, n.y, pfL, pfR);
+      ghost_state(d, d.ebtype[e], time(), xy.x, xy.y, n.x, n.y, pfL, pfR);
     }
     return;
   }
@@ -802,10 +1006,17 @@ __device__ __forceinline__ void face_states(const DevView& d, int e, bool interi
 #pragma unroll
       for (int v = 0; v < 4; v++) {
         const T gradC = pr[v] - pl[v];
+#if FVS_FP64_FAST
+        const T gradL = fma(dl.x, gxl[v], dl.y * gyl[v]);
+        const T gradR = fma(dr.x, gxr[v], dr.y * gyr[v]);
+        pfL[v] = fma(phiL, fma(kh, gradC, omk * gradL), pl[v]);
+        pfR[v] = fma(phiR, fma(nkh, gradC, omk * gradR), pr[v]);
+#else
         const T gradL = dl.x * gxl[v] + dl.y * gyl[v];
         const T gradR = dr.x * gxr[v] + dr.y * gyr[v];
         pfL[v] = pl[v] + phiL * (kh * gradC + omk * gradL);
         pfR[v] = pr[v] + phiR * (nkh * gradC + omk * gradR);
+#endif
       }
     }
   } else {
@@ -814,54 +1025,72 @@ __device__ __forceinline__ void face_states(const DevView& d, int e, bool interi
     for (int v = 0; v < 4; v++) pfL[v] = pl[v] + phiL * (dl.x * gxl[v] + dl.y * gyl[v]);
     // boundary record of the slot: type | case << 4, face centre
     const T2 xy = ld2(d.exy, e);
-    ghost_state(d, d.ebtype[e], time, xy.x, xy.y, n.x, n.y, pfL, pfR);
+    ghost_state(d, d.ebtype[e], time(), xy.x, xy.y, n.x, n.y, pfL, pfR);
   }
 }
 
 // flux * area and ws * area of edge slot e from the cell data in global
-// memory (the edge-flux kernel's loads and arithmetic)
+// memory, in two parts: the slot's cells and geometry, which no kernel of a
+// step writes, then the cell data and the flux
 template <int REC, bool COH>
-__device__ __forceinline__ void flux_compute(const DevView& d, int e, double time, T* flux, T& wsa) {
-  constexpr bool SPEC = REC == REC_SPEC;
-  const T* P = static_cast<const T*>(d.Pv);
-  const T* GX = static_cast<const T*>(d.Gx);
-  const T* GY = static_cast<const T*>(d.Gy);
-  const T* PH = static_cast<const T*>(d.phi);
-  int2 lr = d.ecell[e];
-  lr.x = chk_idx(d.bounds_err, lr.x, 0, d.nc, SITE_EDGE_L);
-  lr.y = chk_idx(d.bounds_err, lr.y, -1, d.nc, SITE_EDGE_R);
-  const T2 n = ld2(d.enrm, e);
-  const T af = static_cast<const T*>(d.earea)[e];
-  const bool interior = lr.y >= 0;
-  T pl[4], gxl[4], gyl[4], pr[4], gxr[4], gyr[4], pfL[4], pfR[4];
-  T phiL = T(1), phiR = T(1);
-  ldc4<COH>(P, lr.x, pl);
-  if (REC != REC_FIRST) {
-    ldc4<COH>(GX, lr.x, gxl);
-    ldc4<COH>(GY, lr.x, gyl);
-    if (!SPEC) phiL = ldc1<COH>(PH, lr.x);
-  }
-  if (interior) {
-    ldc4<COH>(P, lr.y, pr);
+struct FluxItem {
+  int2 lr;
+  T2 n, dl, dr;
+  T af;
+
+  __device__ __forceinline__ void load_static(const DevView& d, int e) {
+    lr = d.ecell[e];
+    lr.x = chk_idx(d.bounds_err, lr.x, 0, d.nc, SITE_EDGE_L);
+    lr.y = chk_idx(d.bounds_err, lr.y, -1, d.nc, SITE_EDGE_R);
+    n = ld2(d.enrm, e);
+    af = static_cast<const T*>(d.earea)[e];
+    dl = {T(0), T(0)};
+    dr = {T(0), T(0)};
     if (REC != REC_FIRST) {
-      ldc4<COH>(GX, lr.y, gxr);
-      ldc4<COH>(GY, lr.y, gyr);
-      if (!SPEC) phiR = ldc1<COH>(PH, lr.y);
+      dl = ld2(d.edL, e);
+      if (lr.y >= 0) dr = ld2(d.edR, e);
     }
   }
-  T2 dl = {T(0), T(0)}, dr = {T(0), T(0)};
-  if (REC != REC_FIRST) {
-    dl = ld2(d.edL, e);
-    if (interior) dr = ld2(d.edR, e);
+  template <class Time>
+  __device__ __forceinline__ void run(const DevView& d, int e, Time time, T* flux, T& wsa) {
+    constexpr bool SPEC = REC == REC_SPEC;
+    const T* P = static_cast<const T*>(d.Pv);
+    const T* GX = static_cast<const T*>(d.Gx);
+    const T* GY = static_cast<const T*>(d.Gy);
+    const T* PH = static_cast<const T*>(d.phi);
+    const bool interior = lr.y >= 0;
+    T pl[4], gxl[4], gyl[4], pr[4], gxr[4], gyr[4], pfL[4], pfR[4];
+    T phiL = T(1), phiR = T(1);
+    ldc4<COH>(P, lr.x, pl);
+    if (REC != REC_FIRST) {
+      ldc4<COH>(GX, lr.x, gxl);
+      ldc4<COH>(GY, lr.x, gyl);
+      if (!SPEC) phiL = ldc1<COH>(PH, lr.x);
+    }
+    if (interior) {
+      ldc4<COH>(P, lr.y, pr);
+      if (REC != REC_FIRST) {
+        ldc4<COH>(GX, lr.y, gxr);
+        ldc4<COH>(GY, lr.y, gyr);
+        if (!SPEC) phiR = ldc1<COH>(PH, lr.y);
+      }
+    }
+    face_states<REC>(d, e, interior, time, n, dl, dr, pl, gxl, gyl, phiL, pr, gxr, gyr, phiR, pfL, pfR);
+    flux_eval(d, pfL, pfR, n, af, flux, wsa);
   }
-  face_states<REC>(d, e, interior, time, n, dl, dr, pl, gxl, gyl, phiL, pr, gxr, gyr, phiR, pfL, pfR);
-  flux_eval(d, pfL, pfR, n, af, flux, wsa);
+};
+
+template <int REC, bool COH, class Time>
+__device__ __forceinline__ void flux_compute(const DevView& d, int e, Time time, T* flux, T& wsa) {
+  FluxItem<REC, COH> f;
+  f.load_static(d, e);
+  f.run(d, e, time, flux, wsa);
 }
 
 // ws_out: also store ws * area (read only by a steady scheme's first stage,
 // for the local time step, and by residual evaluations)
-template <int REC, bool COH>
-__device__ __forceinline__ void flux_item(const DevView& d, int e, double time, bool ws_out = true) {
+template <int REC, bool COH, class Time>
+__device__ __forceinline__ void flux_item(const DevView& d, int e, Time time, bool ws_out = true) {
   T flux[4], wsa;
   flux_compute<REC, COH>(d, e, time, flux, wsa);
   st4(static_cast<T*>(d.eflux), e, flux);
@@ -908,16 +1137,24 @@ __device__ __forceinline__ void flux_range(const DevView& d, int b, int end, int
   if (REC == REC_FIRST) {
     for (int e = b; e < end; e += 2 * stride) flux_first_pair<COH>(d, e, e + stride < end ? e + stride : -1, time);
   } else {
-    for (int e = b; e < end; e += stride) flux_item<REC, COH>(d, e, time);
+    for (int e = b; e < end; e += stride) flux_item<REC, COH>(d, e, [=]() { return time; });
   }
 }
 
 template <int REC>
 __global__ void __launch_bounds__(256) k_flux(const DevView d, double dts, int ws_out) {
-  pdl_wait();
-  pdl_trigger();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < d.nedge) flux_item<REC, false>(d, e, d.tctl[1] + dts, ws_out != 0);
+  FluxItem<REC, false> f;
+  if (e < d.nedge) f.load_static(d, e);
+  pdl_wait();
+  if (d.trig_first) pdl_trigger();
+  if (e < d.nedge) {
+    T flux[4], wsa;
+    f.run(d, e, [&]() { return told_of(d) + dts; }, flux, wsa);
+    st4(static_cast<T*>(d.eflux), e, flux);
+    if (ws_out) static_cast<T*>(d.ews)[e] = wsa;
+  }
+  if (!d.trig_first) pdl_trigger();
 }
 
 // ---------------------------------------------------------------------------
@@ -1599,7 +1836,7 @@ __device__ __forceinline__ void stage_norms(const DevView& d, NormAcc& na, void*
 template <int MODE, bool STRIDE>
 __global__ void __launch_bounds__(256) k_update(const DevView d, const StageParams sp) {
   pdl_wait();
-  pdl_trigger();
+  if (d.trig_first) pdl_trigger();
   NormAcc na;
   if (STRIDE) {
     for (int ic = blockIdx.x * blockDim.x + threadIdx.x; ic < d.nc; ic += gridDim.x * blockDim.x)
@@ -1608,6 +1845,7 @@ __global__ void __launch_bounds__(256) k_update(const DevView d, const StagePara
     const int ic = blockIdx.x * blockDim.x + threadIdx.x;
     if (ic < d.nc) update_item<MODE, false>(d, sp, ic, na);
   }
+  if (!d.trig_first) pdl_trigger();
   __shared__ __align__(16) unsigned char sh[FVS_NORM_SH_BYTES];
   if (sp.last) stage_norms(d, na, sh);
 }
@@ -1698,7 +1936,7 @@ __global__ void __launch_bounds__(256, FVS_MIXED ? 5 : 2) k_tile_stage(const Dev
     __syncthreads();
   }
   // 3. face fluxes
-  const double time = d.tctl[1] + sp.dts;
+  auto time = [&]() { return d.tctl[1] + sp.dts; };
   const int fb = tv.f0[t], nf = tv.f0[t + 1] - fb;
   const T* fg = static_cast<const T*>(tv.fgeo) + 8 * (size_t)fb;
   for (int f = tid; f < nf; f += nthr) {
@@ -1807,7 +2045,7 @@ __global__ void __launch_bounds__(256) k_tile_flux_update(const DevView d, const
   const int t = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
   const int b = tv.c0[t], n = tv.c0[t + 1] - b;
   T* Pout = static_cast<T*>(tv.Pbuf[kout]);
-  const double time = d.tctl[1] + sp.dts;
+  auto time = [&]() { return d.tctl[1] + sp.dts; };
   const int fb = tv.f0[t], nf = tv.f0[t + 1] - fb;
   for (int f = tid; f < nf; f += nthr) {
     T flux[4], wsa;
@@ -1984,7 +2222,7 @@ __global__ void __launch_bounds__(256) k_tile_dma(const DevView d, const TileVie
   }
   __syncthreads();
   // 3. face fluxes
-  const double time = d.tctl[1] + sp.dts;
+  auto time = [&]() { return d.tctl[1] + sp.dts; };
   for (int f = tid; f < nf; f += nthr) {
     const uint32_t lr = sR[f];
     const float* g = sFg + 8 * f;
@@ -2160,14 +2398,11 @@ __global__ void __launch_bounds__(256) k_cvar2pvar(const DevView d) {
   st4(static_cast<T*>(d.Pv), ic, p);
 }
 
-// told = t1 + (istep-1)*dt, src/runge_kutta.f90:207-208
 __global__ void k_begin_step(const DevView d) {
   pdl_wait();
   pdl_trigger();
-  const int istep = d.stepctl[0] + 1;
-  d.tctl[1] = d.tctl[0] + double(istep - 1) * d.dt;
+  d.tctl[1] = told_of(d);
 }
-
 
 // ---------------------------------------------------------------------------
 // persistent kernel: whole RK steps in one cooperative launch
@@ -2545,7 +2780,7 @@ __global__ void __launch_bounds__(256) k_tiles_flux(const DevView d, const Persi
   const int2 tl = p.edge_tiles[blockIdx.x];
   if (ONE) {
     const int e = tl.x + threadIdx.x;
-    if (e < tl.y) flux_item<REC, false>(d, e, told + p.sp[stage].dts);
+    if (e < tl.y) flux_item<REC, false>(d, e, [&]() { return told + p.sp[stage].dts; });
   } else {
     flux_range<REC, false>(d, tl.x + threadIdx.x, tl.y, blockDim.x, told + p.sp[stage].dts);
   }
@@ -2614,30 +2849,40 @@ static cudaError_t launch_tiled_step(const DevView& d, const PersistPlan& p, int
 // ---------------------------------------------------------------------------
 static inline unsigned grid_of(int n) { return (unsigned)((n + 255) / 256); }
 
+// the view of a launch of `grid` blocks of `block` threads, with the place of
+// its pdl_trigger (see there)
+static DevView with_trigger(const DevView& d, unsigned grid, unsigned block) {
+  DevView v = d;
+  v.trig_first = grid <= 76 || (unsigned long long)grid * block >= 200000;
+  return v;
+}
+static inline unsigned grid_for(int n, unsigned block) { return ((unsigned)n + block - 1) / block; }
+
 
 static void launch_begin_step(const DevView& d, cudaStream_t s) { launch_k(k_begin_step, 1, 1, 0, s, d); }
 static void launch_cvar2pvar(const DevView& d, cudaStream_t s) { launch_k(k_cvar2pvar, grid_of(d.nc), 256, 0, s, d); }
 
 static void launch_gradient(const DevView& d, cudaStream_t s) {
   if (d.first_order) return;
-  const unsigned g = grid_of(d.nc);
+  const unsigned b = BLK_GRADIENT, g = grid_for(d.nc, b);
   const bool lim = d.limiter != FVS_LIM_NONE;
   switch (d.grad_method) {
     case FVS_GRAD_LSQ:
-      if (lim) launch_k(k_gradient<FVS_GRAD_LSQ, 1>, g, 256, 0, s, d);
-      else launch_k(k_gradient<FVS_GRAD_LSQ, 0>, g, 256, 0, s, d);
+      if (lim) launch_k(k_gradient<FVS_GRAD_LSQ, 1>, g, b, 0, s, with_trigger(d, g, b));
+      else launch_k(k_gradient<FVS_GRAD_LSQ, 0>, g, b, 0, s, with_trigger(d, g, b));
       break;
-    case FVS_GRAD_GGCB: launch_k(k_gradient<FVS_GRAD_GGCB, 0>, g, 256, 0, s, d); break;
-    default: launch_k(k_gradient<FVS_GRAD_GGNB, 0>, g, 256, 0, s, d); break;
+    case FVS_GRAD_GGCB: launch_k(k_gradient<FVS_GRAD_GGCB, 0>, g, b, 0, s, with_trigger(d, g, b)); break;
+    default: launch_k(k_gradient<FVS_GRAD_GGNB, 0>, g, b, 0, s, with_trigger(d, g, b)); break;
   }
 }
 
 static void launch_flux(const DevView& d, double dts, bool ws_out, cudaStream_t s) {
   const bool spec = !FVS_STRICT && d.khalf == 0.0 && d.omk == 1.0 && d.limiter == FVS_LIM_NONE && !d.first_order;
   const int w = ws_out ? 1 : 0;
-  if (d.first_order) launch_k(k_flux<REC_FIRST>, grid_of(d.nedge), 256, 0, s, d, dts, w);
-  else if (spec) launch_k(k_flux<REC_SPEC>, grid_of(d.nedge), 256, 0, s, d, dts, w);
-  else launch_k(k_flux<REC_GENERAL>, grid_of(d.nedge), 256, 0, s, d, dts, w);
+  const unsigned b = BLK_FLUX, g = grid_for(d.nedge, b);
+  if (d.first_order) launch_k(k_flux<REC_FIRST>, g, b, 0, s, with_trigger(d, g, b), dts, w);
+  else if (spec) launch_k(k_flux<REC_SPEC>, g, b, 0, s, with_trigger(d, g, b), dts, w);
+  else launch_k(k_flux<REC_GENERAL>, g, b, 0, s, with_trigger(d, g, b), dts, w);
 }
 
 // blocks of 256 threads of kernel k resident on the whole device at once
@@ -2659,16 +2904,18 @@ static int update_wave(int mode) {
 
 template <int MODE>
 static void launch_update_mode(const DevView& d, const StageParams& sp, cudaStream_t s) {
-  const unsigned g = grid_of(d.nc);
-  if (!sp.last || d.upd_grid <= 0 || (unsigned)d.upd_grid >= g) {
-    launch_k(k_update<MODE, false>, g, 256, 0, s, d, sp);
+  if (!sp.last || d.upd_grid <= 0 || (unsigned)d.upd_grid >= grid_of(d.nc)) {
+    const unsigned b = BLK_UPDATE, g = grid_for(d.nc, b);
+    DevView dl = with_trigger(d, g, b);
+    dl.nblk_red = (int)g;
+    launch_k(k_update<MODE, false>, g, b, 0, s, dl, sp);
     return;
   }
   // The last stage reduces the norms: one wave of resident blocks walks the
   // cells (grid stride), so that the block-end reduction, fence and counter
   // run once per resident block instead of once per 256 cells, and the last
   // block sums that many partials.
-  DevView dl = d;
+  DevView dl = with_trigger(d, grid_of(d.nc), 256);
   dl.nblk_red = d.upd_grid;
   launch_k(k_update<MODE, true>, (unsigned)d.upd_grid, 256, 0, s, dl, sp);
 }

@@ -131,6 +131,50 @@ struct Layout {
   std::vector<int> st_ptr{0}, st_cell;
   std::vector<T> st_coef, st_w, coef0, coefedg;
   std::vector<int8_t> st_node;
+  // the stencil interleaved over groups of 32 cells (build_ell): per group as
+  // many rows of 32 entries as its longest stencil has
+  std::vector<int> ell_base, ell_cell;
+  std::vector<uint8_t> ell_n;
+  std::vector<T> ell_coef, ell_w;
+
+  // from the CSR rows, entry order kept; places beyond a cell's own entries
+  // hold cell 0 and zeros and are not read
+  bool build_ell() {
+    const int ng = (nc + 31) / 32;
+    const bool node = !st_node.empty();
+    ell_base.assign(1, 0);
+    ell_n.resize(nc);
+    long long total = 0;
+    for (int g = 0; g < ng; g++) {
+      int width = 0;
+      for (int ic = 32 * g; ic < std::min(nc, 32 * g + 32); ic++) {
+        const int n = st_ptr[ic + 1] - st_ptr[ic];
+        if (n > 255) return false;
+        ell_n[ic] = (uint8_t)n;
+        width = std::max(width, n);
+      }
+      total += 32LL * width;
+      if (total > 0x7fffffffLL) return false;
+      ell_base.push_back((int)total);
+    }
+    ell_cell.assign((size_t)total, 0);
+    ell_coef.assign(2 * (size_t)total, T(0));
+    if (!st_w.empty()) ell_w.assign((size_t)total, T(0));
+    for (int ic = 0; ic < nc; ic++)
+      for (int k = st_ptr[ic], at = ell_base[ic / 32] + ic % 32; k < st_ptr[ic + 1]; k++, at += 32) {
+        ell_cell[at] = st_cell[k];
+        if (node) {
+          const T* ce = &coefedg[8 * (size_t)ic + 2 * st_node[k]];
+          ell_coef[2 * (size_t)at] = ce[0] * st_coef[k];
+          ell_coef[2 * (size_t)at + 1] = ce[1] * st_coef[k];
+        } else {
+          ell_coef[2 * (size_t)at] = st_coef[2 * (size_t)k];
+          ell_coef[2 * (size_t)at + 1] = st_coef[2 * (size_t)k + 1];
+        }
+        if (!st_w.empty()) ell_w[at] = st_w[k];
+      }
+    return true;
+  }
 };
 
 // Appends one mesh (case index `cs`) to the layout.  fold_w: LSQ weights
@@ -277,29 +321,39 @@ int append_case(Layout<T>& L, const HostMesh& h, bool fold_w, int cs, std::strin
   return FVS_OK;
 }
 
-// Uploads the mesh arrays of a layout and points the view at them.
+// Uploads the mesh arrays of a layout and points the view at them.  csr: the
+// stencil's CSR rows too (the fused tile stages read them); weights: the LSQ
+// weights (the strict kernels read them).
 template <typename T>
-bool upload_layout(DeviceArena& A, const Layout<T>& L, DevView& d) {
+bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weights) {
+  if (!L.build_ell()) return false;
   bool ok = true;
   double *dvol, *drvol;
   int4* dcf;
   int8_t *dnv, *dsn;
-  int *dsp, *dsc, *deb;
+  int *dsp, *deb, *d_eb, *d_ec;
+  uint8_t* d_en;
   int2* dec;
-  T *t_rvol, *t_eps2, *t_cpos, *t_coef, *t_w, *t_c0, *t_ce, *t_nrm, *t_area, *t_edL, *t_edR, *t_exy;
+  T *t_rvol, *t_eps2, *t_cpos, *t_coef, *t_w = nullptr, *t_c0, *t_ce, *t_ell, *t_nrm, *t_area, *t_edL, *t_edR, *t_exy;
   ok = ok && A.upload(dvol, L.vol) && A.upload(drvol, L.rvol) && A.upload(dcf, L.cf) && A.upload(dnv, L.nvrt);
-  ok = ok && A.upload(dsp, L.st_ptr) && A.upload(dsc, L.st_cell) && A.upload(dsn, L.st_node) && A.upload(dec, L.ecell);
+  ok = ok && A.upload(d_eb, L.ell_base) && A.upload(d_en, L.ell_n) && A.upload(d_ec, L.ell_cell) && A.upload(t_ell, L.ell_coef);
+  ok = ok && A.upload(dec, L.ecell);
   ok = ok && A.upload(deb, L.ebtype) && A.upload(t_rvol, L.rvolT) && A.upload(t_eps2, L.eps2);
-  ok = ok && A.upload(t_cpos, L.cpos) && A.upload(t_coef, L.st_coef) && A.upload(t_w, L.st_w);
-  ok = ok && A.upload(t_c0, L.coef0) && A.upload(t_ce, L.coefedg) && A.upload(t_nrm, L.enrm) && A.upload(t_area, L.earea);
+  ok = ok && A.upload(t_cpos, L.cpos) && (!weights || A.upload(t_w, L.ell_w));
+  ok = ok && A.upload(t_c0, L.coef0) && A.upload(t_nrm, L.enrm) && A.upload(t_area, L.earea);
   ok = ok && A.upload(t_edL, L.edL) && A.upload(t_edR, L.edR) && A.upload(t_exy, L.exy);
+  if (ok && csr) {
+    ok = A.upload(dsp, L.st_ptr) && A.upload(t_coef, L.st_coef) && A.upload(dsn, L.st_node) && A.upload(t_ce, L.coefedg);
+    d.st_ptr = dsp; d.st_coef = t_coef; d.st_node = dsn; d.coefedg = t_ce;
+  }
   if (!ok) return false;
   d.nc = L.nc;
   d.nint = L.nint;
   d.nedge = L.ne;
-  d.vol = dvol; d.rvol = drvol; d.cflist = dcf; d.nvrt = dnv; d.st_ptr = dsp; d.st_cell = dsc; d.st_node = dsn;
-  d.ecell = dec; d.ebtype = deb; d.volT = t_rvol; d.eps2 = t_eps2; d.cpos = t_cpos; d.st_coef = t_coef; d.st_w = t_w;
-  d.coef0 = t_c0; d.coefedg = t_ce; d.enrm = t_nrm; d.earea = t_area; d.edL = t_edL; d.edR = t_edR; d.exy = t_exy;
+  d.vol = dvol; d.rvol = drvol; d.cflist = dcf; d.nvrt = dnv;
+  d.ell_base = d_eb; d.ell_n = d_en; d.ell_cell = d_ec; d.ell_coef = t_ell; d.ell_w = t_w;
+  d.ecell = dec; d.ebtype = deb; d.volT = t_rvol; d.eps2 = t_eps2; d.cpos = t_cpos;
+  d.coef0 = t_c0; d.enrm = t_nrm; d.earea = t_area; d.edL = t_edL; d.edR = t_edR; d.exy = t_exy;
   return true;
 }
 
