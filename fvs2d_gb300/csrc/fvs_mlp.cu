@@ -9,6 +9,11 @@
 // mma.sync m16n8k16 kernel below (kept as the comparison engine).
 // Training: minibatch Adam on the mean squared error.
 //
+// With tcgen05 a training step is a gather, one GEMM per layer forward (the last
+// one with the loss and its gradient as epilogue), one per layer backward (GELU'
+// as epilogue), one launch for all weight and bias gradients and one that adds
+// their partial sums and applies Adam: 2 (depth + 1) + 2 launches.
+//
 // GEMM convention: C[m][n] = sum_k A(m,k) B(n,k) (+ bias[n]); each operand is
 // either K-major (row m at A + m*lda) or stored transposed (element (m,k) at
 // A + k*lda + m), which covers the forward pass (X W^T), the input gradient
@@ -148,32 +153,31 @@ __global__ void k_f32_to_bf16(const float* __restrict__ x, bf16* __restrict__ y,
   if (i < n) y[i] = __float2bfloat16(x[i]);
 }
 
-// rows of the dataset selected by idx, padded to ld columns, as BF16
+// rows of the dataset selected by idx (null: all), padded to ld columns, as BF16
 __global__ void k_gather_rows(const float* __restrict__ x, int ncol, const int* __restrict__ idx, int n, bf16* __restrict__ out,
                               int ld) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * ld) return;
   const int r = i / ld, c = i % ld;
-  out[i] = __float2bfloat16(c < ncol ? x[(size_t)idx[r] * ncol + c] : 0.f);
+  out[i] = __float2bfloat16(c < ncol ? x[(size_t)(idx ? idx[r] : r) * ncol + c] : 0.f);
 }
 
-__global__ void k_gather_rows_f32(const float* __restrict__ x, int ncol, const int* __restrict__ idx, int n, float* __restrict__ out) {
+// the first nout columns of Y
+__global__ void k_columns(const float* __restrict__ Y, int ldy, int n, int nout, float* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * ncol) return;
-  const int r = i / ncol, c = i % ncol;
-  out[i] = x[(size_t)idx[r] * ncol + c];
+  if (i < n * nout) out[i] = Y[(size_t)(i / nout) * ldy + i % nout];
 }
 
-// dY = 2 (Y - T) / (n * nout) as BF16 (ld = ldg), squared error summed into loss
-__global__ void k_mse(const float* __restrict__ Y, int ldy, const float* __restrict__ T, int n, int nout, bf16* __restrict__ dY,
-                      int ldg, float* __restrict__ loss_acc) {
+// dY = 2 (Y - T[idx]) / (n * nout) as BF16 (ld = ldg), squared error summed into loss
+__global__ void k_mse(const float* __restrict__ Y, int ldy, const float* __restrict__ T, const int* __restrict__ idx, int n,
+                      int nout, bf16* __restrict__ dY, int ldg, float* __restrict__ loss_acc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   float e2 = 0.f;
   if (i < n * ldg) {
     const int r = i / ldg, c = i % ldg;
     float d = 0.f;
     if (c < nout) {
-      d = Y[(size_t)r * ldy + c] - T[(size_t)r * nout + c];
+      d = Y[(size_t)r * ldy + c] - T[(size_t)(idx ? idx[r] : r) * nout + c];
       e2 = d * d;
     }
     dY[i] = __float2bfloat16(2.f * d / float(n * nout));
@@ -239,21 +243,46 @@ struct fvs_mlp {
   float* am = nullptr;               // Adam moments
   float* av = nullptr;
   bf16* wb = nullptr;                // BF16 copy of the weights
-  int cap = 0;                       // rows of the activation buffers
-  std::vector<bf16*> act;            // act[l]: input of layer l, [cap][din[l]]
-  std::vector<float*> pre;           // pre[l]: layer output before GELU, [cap][dout[l]]
-  bf16* dz = nullptr;                // [cap][max dim]
-  bf16* dz2 = nullptr;
-  float* da = nullptr;               // [cap][max dim]
+  // workspaces, grown to the largest call so far and kept until the handle goes
+  template <typename V>
+  struct Buf {
+    V* p = nullptr;
+    size_t cap = 0;
+    bool grow(size_t n) {
+      if (n <= cap) return true;
+      if (p) cudaFree(p);
+      p = nullptr;
+      cap = 0;
+      if (cudaMalloc(&p, sizeof(V) * n) != cudaSuccess) {
+        cudaGetLastError();  // reported to the caller as FVS_ERR_NOMEM
+        p = nullptr;
+        return false;
+      }
+      cap = n;
+      return true;
+    }
+    Buf() = default;
+    Buf(const Buf&) = delete;
+    Buf& operator=(const Buf&) = delete;
+    Buf(Buf&& o) noexcept : p(o.p), cap(o.cap) { o.p = nullptr; o.cap = 0; }
+    ~Buf() { if (p) cudaFree(p); }
+  };
+  std::vector<Buf<bf16>> act;        // act[l]: input of layer l, [rows][din[l]]
+  std::vector<Buf<float>> pre;       // pre[l]: layer output before GELU, [rows][dout[l]] (training)
+  std::vector<Buf<bf16>> dz;         // dz[l]: loss gradient of pre[l] (training)
+  Buf<float> part;                   // partial sums of the parameter gradients
+  Buf<float> da;                     // mma.sync engine: gradient of a layer's input
+  Buf<float> out;                    // mma.sync engine: last layer's output; prediction rows
+  Buf<float> data_x, data_y;         // the call's rows on the device
+  Buf<int> data_idx;
   float* loss = nullptr;
   int* gemm_err = nullptr;           // set by a tcgen05 GEMM whose bounded wait expired
-  float* split_ws = nullptr;         // split-K partial sums of the tcgen05 GEMM
-  size_t split_cap = 0;              // floats
   int engine = 0;                    // 0: tcgen05, 1: mma.sync
   int step = 0;
   std::vector<void*> owned;
 
   ~fvs_mlp() {
+    if (stream) cudaStreamSynchronize(stream);
     for (void* p : owned) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -269,100 +298,212 @@ struct fvs_mlp {
     owned.push_back(p);
     return static_cast<V*>(p);
   }
-  bool ensure_cap(int rows) {
-    if (rows <= cap) return true;
-    const int maxd = std::max(*std::max_element(din.begin(), din.end()), *std::max_element(dout.begin(), dout.end()));
-    act.assign(nl + 1, nullptr);
-    pre.assign(nl, nullptr);
-    for (int l = 0; l <= nl; l++) act[l] = dalloc<bf16>((size_t)rows * (l < nl ? din[l] : dout[nl - 1]));
-    for (int l = 0; l < nl; l++) pre[l] = dalloc<float>((size_t)rows * dout[l]);
-    dz = dalloc<bf16>((size_t)rows * maxd);
-    dz2 = dalloc<bf16>((size_t)rows * maxd);
-    da = dalloc<float>((size_t)rows * maxd);
-    for (int l = 0; l <= nl; l++) if (!act[l]) return false;
-    for (int l = 0; l < nl; l++) if (!pre[l]) return false;
-    if (!dz || !dz2 || !da) return false;
-    cap = rows;
-    return true;
+  // layer buffers for `rows` rows; train: those of the backward pass too
+  bool ensure_rows(size_t rows, bool train) {
+    act.resize(nl);
+    pre.resize(nl);
+    dz.resize(nl);
+    const size_t maxd = (size_t)std::max(*std::max_element(din.begin(), din.end()), *std::max_element(dout.begin(), dout.end()));
+    bool ok = true;
+    for (int l = 0; l < nl && ok; l++) {
+      ok = act[l].grow(rows * din[l]);
+      if (ok && train) ok = dz[l].grow(rows * dout[l]);
+      if (ok && (engine == 1 || (train && l < nl - 1))) ok = pre[l].grow(rows * dout[l]);
+    }
+    if (ok && engine == 1 && train) ok = da.grow(rows * maxd);
+    return ok;
   }
 };
 
 namespace {
 
+// launch in stream order, the kernel's set-up beside its predecessor's tail
+// (each waits for it with griddepcontrol.wait before it reads or writes)
+template <typename... KArgs, typename... Args>
+void launch_tc(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <bool A_KM, bool B_KM, int OUT>
+void gemm_tc(fvs_mlp* m, const tc::GemmArgs& a) {
+  const dim3 grid((unsigned)((a.N + tc::BN - 1) / tc::BN), (unsigned)((a.M + tc::BM - 1) / tc::BM));
+  // With more tiles than two per SM the epilogues of some CTAs run beside the
+  // loads of others, and four CTAs with two stages each beat two with four
+  // (65,536 x 256 x 256 with GELU: 68 / 79 us); below that a CTA has only its
+  // own blocks in flight.
+  if (grid.x * grid.y > 304)
+    launch_tc(tc::k_gemm_tc<A_KM, B_KM, OUT, 2>, grid, tc::THREADS, tc::smem_bytes(2), m->stream, a, m->gemm_err);
+  else
+    launch_tc(tc::k_gemm_tc<A_KM, B_KM, OUT, 4>, grid, tc::THREADS, tc::smem_bytes(4), m->stream, a, m->gemm_err);
+}
+
 template <bool A_KM, bool B_KM>
-void gemm(fvs_mlp* m, const bf16* A, int lda, const bf16* B, int ldb, int M, int N, int K, int epi,
-          const float* bias, float* C, int ldc, bf16* Cact, int ldact) {
-  if (m->engine == 0) {
-    const int tiles = ((N + tc::BN - 1) / tc::BN) * ((M + tc::BM - 1) / tc::BM);
-    const int nk = (K + tc::BK - 1) / tc::BK;
-    int nsplit = 1;
-    if (epi == EPI_F32 && C && !Cact && tiles < 64 && nk >= 4) {
-      // few output tiles and a long K (the weight gradient, K = batch rows):
-      // split K so that about one CTA per SM works, then add the partials
-      const int want = std::max(1, 148 / tiles);
-      const int per = std::max(1, (nk + want - 1) / want);
-      nsplit = (nk + per - 1) / per;
-      const size_t need = (size_t)nsplit * M * ldc;
-      if (nsplit > 1 && need > m->split_cap) {
-        float* w = m->dalloc<float>(need);
-        if (w) {
-          m->split_ws = w;
-          m->split_cap = need;
-        } else {
-          nsplit = 1;
-        }
-      }
-    }
-    dim3 grid((unsigned)((N + tc::BN - 1) / tc::BN), (unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)nsplit);
-    const size_t stride = (size_t)M * ldc;
-    float* out = nsplit > 1 ? m->split_ws : C;
-    tc::k_gemm_tc<A_KM, B_KM><<<grid, tc::THREADS, tc::SMEM_BYTES, m->stream>>>(A, lda, B, ldb, M, N, K, epi, bias,
-                                                                              out, ldc, Cact, ldact, m->gemm_err,
-                                                                              stride);
-    if (nsplit > 1)
-      tc::k_sum_splits<<<nblk((size_t)M * N), 256, 0, m->stream>>>(m->split_ws, nsplit, stride, M, N, ldc, C);
-    return;
-  }
+void gemm_mma(fvs_mlp* m, const bf16* A, int lda, const bf16* B, int ldb, int M, int N, int K, int epi,
+              const float* bias, float* C, int ldc, bf16* Cact, int ldact) {
   dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM));
   k_gemm<A_KM, B_KM><<<grid, GEMM_THREADS, 0, m->stream>>>(A, lda, B, ldb, M, N, K, epi, bias, C, ldc, Cact, ldact);
 }
 
-// the tcgen05 GEMM uses 64 KB of dynamic shared memory
+// dynamic shared memory of the tcgen05 GEMMs
+template <class Kernel>
+bool tc_smem(Kernel k, int stages) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::smem_bytes(stages)) == cudaSuccess;
+}
+template <bool A_KM, bool B_KM, int OUT>
+bool tc_smem_both() {
+  return tc_smem(tc::k_gemm_tc<A_KM, B_KM, OUT, 2>, 2) && tc_smem(tc::k_gemm_tc<A_KM, B_KM, OUT, 4>, 4);
+}
 bool tc_gemm_setup() {
-  const int b = tc::SMEM_BYTES;
-  return cudaFuncSetAttribute(tc::k_gemm_tc<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b) == cudaSuccess &&
-         cudaFuncSetAttribute(tc::k_gemm_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b) == cudaSuccess &&
-         cudaFuncSetAttribute(tc::k_gemm_tc<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b) == cudaSuccess &&
-         cudaFuncSetAttribute(tc::k_gemm_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b) == cudaSuccess;
+  return tc_smem_both<true, true, tc::OUT_GELU>() && tc_smem_both<true, true, tc::OUT_PRED>() &&
+         tc_smem_both<true, true, tc::OUT_MSE>() && tc_smem_both<true, false, tc::OUT_DGELU>() && tc_smem(tc::k_grads, 2);
 }
 
 void refresh_bf16(fvs_mlp* m) { k_f32_to_bf16<<<nblk(m->nparam), 256, 0, m->stream>>>(m->w, m->wb, m->nparam); }
 
-// forward over n rows already in act[0]; outputs pre[nl-1]
-void forward(fvs_mlp* m, int n) {
-  for (int l = 0; l < m->nl; l++) {
-    const bool last = l == m->nl - 1;
-    gemm<true, true>(m, m->act[l], m->din[l], m->wb + m->woff[l], m->din[l], n, m->dout[l], m->din[l],
-                     last ? EPI_BIAS_F32 : EPI_BIAS_GELU, m->w + m->boff[l], m->pre[l], m->dout[l], last ? nullptr : m->act[l + 1],
-                     m->dout[l]);
+// Forward over n rows already in act[0].  Training (y given): the loss
+// gradient of the last layer into dz, the squared errors against rows idx of
+// y (null: the first n) added to loss, the hidden layers' pre-activations
+// kept.  Otherwise the output's n_out columns into pred.
+void forward(fvs_mlp* m, int n, const float* y, const int* idx, float* pred) {
+  const int last = m->nl - 1;
+  for (int l = 0; l <= last; l++) {
+    const int di = m->din[l], dn = m->dout[l];
+    const bf16* W = m->wb + m->woff[l];
+    const float* bias = m->w + m->boff[l];
+    if (m->engine == 1) {
+      gemm_mma<true, true>(m, m->act[l].p, di, W, di, n, dn, di, l == last ? EPI_BIAS_F32 : EPI_BIAS_GELU, bias,
+                           m->pre[l].p, dn, l == last ? nullptr : m->act[l + 1].p, dn);
+      continue;
+    }
+    tc::GemmArgs a = {};
+    a.A = m->act[l].p; a.lda = di;
+    a.B = W; a.ldb = di;
+    a.M = n; a.N = dn; a.K = di;
+    a.bias = bias;
+    if (l < last) {
+      a.C = y ? m->pre[l].p : nullptr;
+      a.H = m->act[l + 1].p;
+      gemm_tc<true, true, tc::OUT_GELU>(m, a);
+    } else if (y) {
+      a.H = m->dz[l].p;
+      a.T = y; a.idx = idx; a.nt = m->n_out; a.loss = m->loss;
+      gemm_tc<true, true, tc::OUT_MSE>(m, a);
+    } else {
+      a.C = pred; a.nt = m->n_out;
+      gemm_tc<true, true, tc::OUT_PRED>(m, a);
+    }
   }
+  if (m->engine != 1) return;
+  if (y)
+    k_mse<<<nblk((size_t)n * m->out_pad), 256, 0, m->stream>>>(m->pre[last].p, m->out_pad, y, idx, n, m->n_out,
+                                                              m->dz[last].p, m->out_pad, m->loss);
+  else
+    k_columns<<<nblk((size_t)n * m->n_out), 256, 0, m->stream>>>(m->pre[last].p, m->out_pad, n, m->n_out, pred);
 }
 
-// backward from dY (BF16, [n][out_pad]) in dz; gradients into g
-void backward(fvs_mlp* m, int n) {
-  bf16* dcur = m->dz;
-  bf16* dnext = m->dz2;
+// The runs of K blocks that the parameter gradients are summed in (tc::k_grads).
+// A layer's runs are as many as make about one 128 x 128 tile per SM: their number
+// fixes the order of the FP32 sums, and with it the training's trajectory (runs
+// five times longer, added in the same order, moved a weight by 5e-5 of the
+// weights' norm after 32 steps, through BF16 roundings that fell the other way).
+// A CTA takes as many consecutive runs as leave the launch in one wave of four
+// CTAs per SM.
+bool grad_plan(fvs_mlp* m, int rows, tc::GradPlan& p) {
+  p = tc::GradPlan();
+  p.nl = m->nl;
+  p.rows = rows;
+  const int nk = (rows + tc::BK - 1) / tc::BK;
+  size_t off = 0;
+  long long tile_runs = 0;
+  for (int l = 0; l < m->nl; l++) {
+    tc::GradLayer& g = p.l[l];
+    g.dZ = m->dz[l].p; g.X = m->act[l].p;
+    g.din = m->din[l]; g.dout = m->dout[l];
+    g.tiles_n = (g.din + tc::BN - 1) / tc::BN;
+    g.tiles = g.tiles_n * ((g.dout + tc::BM - 1) / tc::BM);
+    const int square = ((g.din + 127) / 128) * ((g.dout + 127) / 128);
+    g.per = nk;
+    if (square < 64 && nk >= 4) {
+      const int want = std::max(1, 148 / square);
+      g.per = std::max(1, (nk + want - 1) / want);
+    }
+    g.nsplit = (nk + g.per - 1) / g.per;
+    tile_runs += (long long)g.tiles * g.nsplit;
+    g.w0 = m->woff[l]; g.b0 = m->boff[l];
+    g.part = off;
+    off += (size_t)g.nsplit * g.din * g.dout + (size_t)g.dout;
+  }
+  int bias_ctas = 0;
+  for (int l = 0; l < m->nl; l++) bias_ctas += (m->dout[l] + tc::BIAS_COLS - 1) / tc::BIAS_COLS;
+  const int room = std::max(304, 608 - bias_ctas);
+  p.runs = (int)std::max<long long>(1, (tile_runs + room - 1) / room);
+  for (int l = 0; l < m->nl; l++) {
+    tc::GradLayer& g = p.l[l];
+    g.cta0 = p.gemm_ctas;
+    p.gemm_ctas += g.tiles * ((g.nsplit + p.runs - 1) / p.runs);
+  }
+  p.ctas = p.gemm_ctas;
+  for (int l = 0; l < m->nl; l++) {
+    p.l[l].bias0 = p.ctas;
+    p.ctas += (m->dout[l] + tc::BIAS_COLS - 1) / tc::BIAS_COLS;
+  }
+  return m->part.grow(off);
+}
+
+// Backward from dz of the last layer: the other layers' dz, then the
+// parameter gradients: into g, or (adam) straight into Adam's step.
+bool backward(fvs_mlp* m, int n, const tc::AdamArgs* adam) {
   for (int l = m->nl - 1; l >= 0; l--) {
     const int di = m->din[l], dn = m->dout[l];
-    // dW_l[n][k] = sum_m dZ[m][n] act_l[m][k]
-    gemm<false, false>(m, dcur, dn, m->act[l], di, dn, di, n, EPI_F32, nullptr, m->g + m->woff[l], di, nullptr, 0);
-    k_colsum<<<(dn + 31) / 32, dim3(32, 32), 0, m->stream>>>(dcur, n, dn, dn, m->g + m->boff[l]);
+    if (m->engine == 1) {
+      // dW_l[n][k] = sum_m dZ[m][n] act_l[m][k]
+      gemm_mma<false, false>(m, m->dz[l].p, dn, m->act[l].p, di, dn, di, n, EPI_F32, nullptr, m->g + m->woff[l], di, nullptr, 0);
+      k_colsum<<<(dn + 31) / 32, dim3(32, 32), 0, m->stream>>>(m->dz[l].p, n, dn, dn, m->g + m->boff[l]);
+    }
     if (l == 0) break;
-    // dA_{l}[m][k] = sum_n dZ[m][n] W_l[n][k]; dZ_{l-1} = dA * gelu'(pre_{l-1})
-    gemm<true, false>(m, dcur, dn, m->wb + m->woff[l], di, n, di, dn, EPI_F32, nullptr, m->da, di, nullptr, 0);
-    k_gelu_back<<<nblk((size_t)n * di), 256, 0, m->stream>>>(m->da, m->pre[l - 1], dnext, (size_t)n * di);
-    std::swap(dcur, dnext);
+    // dA_l[m][k] = sum_n dZ[m][n] W_l[n][k]; dZ_{l-1} = dA * gelu'(pre_{l-1})
+    if (m->engine == 1) {
+      gemm_mma<true, false>(m, m->dz[l].p, dn, m->wb + m->woff[l], di, n, di, dn, EPI_F32, nullptr, m->da.p, di, nullptr, 0);
+      k_gelu_back<<<nblk((size_t)n * di), 256, 0, m->stream>>>(m->da.p, m->pre[l - 1].p, m->dz[l - 1].p, (size_t)n * di);
+    } else {
+      tc::GemmArgs a = {};
+      a.A = m->dz[l].p; a.lda = dn;
+      a.B = m->wb + m->woff[l]; a.ldb = di;
+      a.M = n; a.N = di; a.K = dn;
+      a.Z = m->pre[l - 1].p;
+      a.H = m->dz[l - 1].p;
+      gemm_tc<true, false, tc::OUT_DGELU>(m, a);
+    }
   }
+  if (m->engine == 1) {
+    if (adam) {
+      k_adam<<<nblk(m->nparam), 256, 0, m->stream>>>(m->w, m->g, m->am, m->av, m->nparam, adam->lr, adam->b1, adam->b2,
+                                                     adam->eps, adam->bc1, adam->bc2);
+      refresh_bf16(m);
+    }
+    return true;
+  }
+  tc::GradPlan p;
+  if (!grad_plan(m, n, p)) return false;
+  launch_tc(tc::k_grads, dim3((unsigned)p.ctas), tc::THREADS, tc::smem_bytes(2), m->stream, p,
+            m->part.p, m->gemm_err);
+  if (adam)
+    launch_tc(tc::k_finish_grads<true>, dim3(nblk(m->nparam)), 256, 0, m->stream, p, (const float*)m->part.p, m->nparam,
+              m->g, m->w, m->am, m->av, m->wb, *adam);
+  else
+    launch_tc(tc::k_finish_grads<false>, dim3(nblk(m->nparam)), 256, 0, m->stream, p, (const float*)m->part.p, m->nparam,
+              m->g, m->w, m->am, m->av, m->wb, tc::AdamArgs());
+  return true;
 }
 
 int check(fvs_mlp* m, const char* where) {
@@ -510,23 +651,16 @@ int fvs_mlp_set_params(fvs_mlp* m, const float* src, int64_t n) {
 // loss and parameter gradients of one batch (no update), for checking
 int fvs_mlp_loss_grad(fvs_mlp* m, const float* x, const float* y, int32_t n, float* loss, float* grads) {
   if (!m || !x || !y || n <= 0) return FVS_ERR_INVALID;
-  if (!m->ensure_cap(n)) return m->fail(FVS_ERR_NOMEM, "activation allocation");
-  float* dx = m->dalloc<float>((size_t)n * m->n_in);
-  float* dy = m->dalloc<float>((size_t)n * m->n_out);
-  int* di = m->dalloc<int>(n);
-  if (!dx || !dy || !di) return m->fail(FVS_ERR_NOMEM, "batch allocation");
-  std::vector<int> idx(n);
-  for (int i = 0; i < n; i++) idx[i] = i;
-  cudaMemcpy(dx, x, 4 * (size_t)n * m->n_in, cudaMemcpyHostToDevice);
-  cudaMemcpy(dy, y, 4 * (size_t)n * m->n_out, cudaMemcpyHostToDevice);
-  cudaMemcpy(di, idx.data(), 4 * (size_t)n, cudaMemcpyHostToDevice);
-  k_gather_rows<<<nblk((size_t)n * m->in_pad), 256, 0, m->stream>>>(dx, m->n_in, di, n, m->act[0], m->in_pad);
-  forward(m, n);
+  if (!m->ensure_rows(n, true)) return m->fail(FVS_ERR_NOMEM, "activation allocation");
+  if (!m->data_x.grow((size_t)n * m->n_in) || !m->data_y.grow((size_t)n * m->n_out))
+    return m->fail(FVS_ERR_NOMEM, "batch allocation");
+  cudaMemcpyAsync(m->data_x.p, x, 4 * (size_t)n * m->n_in, cudaMemcpyHostToDevice, m->stream);
+  cudaMemcpyAsync(m->data_y.p, y, 4 * (size_t)n * m->n_out, cudaMemcpyHostToDevice, m->stream);
   cudaMemsetAsync(m->loss, 0, 4, m->stream);
-  k_mse<<<nblk((size_t)n * m->out_pad), 256, 0, m->stream>>>(m->pre[m->nl - 1], m->out_pad, dy, n, m->n_out, m->dz,
-                                                            m->out_pad, m->loss);
-  cudaMemsetAsync(m->g, 0, 4 * m->nparam, m->stream);
-  backward(m, n);
+  if (m->engine == 1) cudaMemsetAsync(m->g, 0, 4 * m->nparam, m->stream);
+  k_gather_rows<<<nblk((size_t)n * m->in_pad), 256, 0, m->stream>>>(m->data_x.p, m->n_in, nullptr, n, m->act[0].p, m->in_pad);
+  forward(m, n, m->data_y.p, nullptr, nullptr);
+  if (!backward(m, n, nullptr)) return m->fail(FVS_ERR_NOMEM, "gradient workspace");
   int rc = check(m, "loss_grad");
   if (rc) return rc;
   float l = 0.f;
@@ -545,35 +679,33 @@ int fvs_mlp_train(fvs_mlp* m, const float* x, const float* y, int64_t n, int32_t
                   uint64_t seed, float* loss_per_epoch) {
   if (!m || !x || !y || n <= 0 || batch <= 0 || epochs <= 0 || n > (int64_t)1 << 31) return FVS_ERR_INVALID;
   batch = (int)std::min<int64_t>(batch, n);
-  if (!m->ensure_cap(batch)) return m->fail(FVS_ERR_NOMEM, "activation allocation");
-  float* dx = m->dalloc<float>((size_t)n * m->n_in);
-  float* dy = m->dalloc<float>((size_t)n * m->n_out);
-  float* ty = m->dalloc<float>((size_t)batch * m->n_out);
-  int* didx = m->dalloc<int>(n);
-  if (!dx || !dy || !ty || !didx) return m->fail(FVS_ERR_NOMEM, "dataset allocation");
-  cudaMemcpy(dx, x, 4 * (size_t)n * m->n_in, cudaMemcpyHostToDevice);
-  cudaMemcpy(dy, y, 4 * (size_t)n * m->n_out, cudaMemcpyHostToDevice);
+  if (!m->ensure_rows(batch, true)) return m->fail(FVS_ERR_NOMEM, "activation allocation");
+  if (!m->data_x.grow((size_t)n * m->n_in) || !m->data_y.grow((size_t)n * m->n_out) || !m->data_idx.grow((size_t)n))
+    return m->fail(FVS_ERR_NOMEM, "dataset allocation");
+  cudaMemcpyAsync(m->data_x.p, x, 4 * (size_t)n * m->n_in, cudaMemcpyHostToDevice, m->stream);
+  cudaMemcpyAsync(m->data_y.p, y, 4 * (size_t)n * m->n_out, cudaMemcpyHostToDevice, m->stream);
   std::vector<int> idx(n);
   std::mt19937_64 rng(seed);
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  for (int ep = 0; ep < epochs; ep++) {
+  auto shuffle = [&]() {
     for (int64_t i = 0; i < n; i++) idx[i] = (int)i;
     std::shuffle(idx.begin(), idx.end(), rng);
-    cudaMemcpyAsync(didx, idx.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, m->stream);
+  };
+  shuffle();
+  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  for (int ep = 0; ep < epochs; ep++) {
+    // (pageable: copied out of idx when the call returns)
+    cudaMemcpyAsync(m->data_idx.p, idx.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, m->stream);
     cudaMemsetAsync(m->loss, 0, 4, m->stream);
     for (int64_t s0 = 0; s0 + batch <= n; s0 += batch) {
-      const int* bi = didx + s0;
-      k_gather_rows<<<nblk((size_t)batch * m->in_pad), 256, 0, m->stream>>>(dx, m->n_in, bi, batch, m->act[0], m->in_pad);
-      k_gather_rows_f32<<<nblk((size_t)batch * m->n_out), 256, 0, m->stream>>>(dy, m->n_out, bi, batch, ty);
-      forward(m, batch);
-      k_mse<<<nblk((size_t)batch * m->out_pad), 256, 0, m->stream>>>(m->pre[m->nl - 1], m->out_pad, ty, batch, m->n_out, m->dz,
-                                                                      m->out_pad, m->loss);
-      backward(m, batch);
+      const int* bi = m->data_idx.p + s0;
+      k_gather_rows<<<nblk((size_t)batch * m->in_pad), 256, 0, m->stream>>>(m->data_x.p, m->n_in, bi, batch, m->act[0].p,
+                                                                            m->in_pad);
+      forward(m, batch, m->data_y.p, bi, nullptr);
       m->step++;
-      k_adam<<<nblk(m->nparam), 256, 0, m->stream>>>(m->w, m->g, m->am, m->av, m->nparam, lr, b1, b2, eps,
-                                                     1.f - std::pow(b1, (float)m->step), 1.f - std::pow(b2, (float)m->step));
-      refresh_bf16(m);
+      const tc::AdamArgs ad = {lr, b1, b2, eps, 1.f - std::pow(b1, (float)m->step), 1.f - std::pow(b2, (float)m->step)};
+      if (!backward(m, batch, &ad)) return m->fail(FVS_ERR_NOMEM, "gradient workspace");
     }
+    if (ep + 1 < epochs) shuffle();  // the next epoch's order, beside this epoch's steps
     int rc = check(m, "train");
     if (rc) return rc;
     if (loss_per_epoch) {
@@ -588,26 +720,17 @@ int fvs_mlp_train(fvs_mlp* m, const float* x, const float* y, int64_t n, int32_t
 int fvs_mlp_predict(fvs_mlp* m, const float* x, int64_t n, float* y) {
   if (!m || !x || !y || n <= 0) return FVS_ERR_INVALID;
   const int chunk = (int)std::min<int64_t>(n, 65536);
-  if (!m->ensure_cap(chunk)) return m->fail(FVS_ERR_NOMEM, "activation allocation");
-  float* dx = m->dalloc<float>((size_t)chunk * m->n_in);
-  int* di = m->dalloc<int>(chunk);
-  if (!dx || !di) return m->fail(FVS_ERR_NOMEM, "batch allocation");
-  std::vector<int> idx(chunk);
-  for (int i = 0; i < chunk; i++) idx[i] = i;
-  cudaMemcpy(di, idx.data(), 4 * (size_t)chunk, cudaMemcpyHostToDevice);
-  std::vector<float> out((size_t)chunk * m->out_pad);
+  if (!m->ensure_rows(chunk, false)) return m->fail(FVS_ERR_NOMEM, "activation allocation");
+  if (!m->data_x.grow((size_t)chunk * m->n_in) || !m->out.grow((size_t)chunk * m->n_out))
+    return m->fail(FVS_ERR_NOMEM, "batch allocation");
   for (int64_t s0 = 0; s0 < n; s0 += chunk) {
     const int c = (int)std::min<int64_t>(chunk, n - s0);
-    cudaMemcpyAsync(dx, x + s0 * m->n_in, 4 * (size_t)c * m->n_in, cudaMemcpyHostToDevice, m->stream);
-    k_gather_rows<<<nblk((size_t)c * m->in_pad), 256, 0, m->stream>>>(dx, m->n_in, di, c, m->act[0], m->in_pad);
-    forward(m, c);
-    cudaMemcpyAsync(out.data(), m->pre[m->nl - 1], 4 * (size_t)c * m->out_pad, cudaMemcpyDeviceToHost, m->stream);
-    int rc = check(m, "predict");
-    if (rc) return rc;
-    for (int r = 0; r < c; r++)
-      for (int k = 0; k < m->n_out; k++) y[(s0 + r) * m->n_out + k] = out[(size_t)r * m->out_pad + k];
+    cudaMemcpyAsync(m->data_x.p, x + s0 * m->n_in, 4 * (size_t)c * m->n_in, cudaMemcpyHostToDevice, m->stream);
+    k_gather_rows<<<nblk((size_t)c * m->in_pad), 256, 0, m->stream>>>(m->data_x.p, m->n_in, nullptr, c, m->act[0].p, m->in_pad);
+    forward(m, c, nullptr, nullptr, m->out.p);
+    cudaMemcpyAsync(y + s0 * m->n_out, m->out.p, 4 * (size_t)c * m->n_out, cudaMemcpyDeviceToHost, m->stream);
   }
-  return FVS_OK;
+  return check(m, "predict");
 }
 
 }  // extern "C"

@@ -1,25 +1,28 @@
 // fvs_tcgemm.cuh — BF16 GEMM on the 5th-generation tensor cores (tcgen05),
 // FP32 accumulation in tensor memory:  C[m][n] = sum_k A(m,k) B(n,k).
 //
-// Operands are K-major (row m at A + m*lda) or stored transposed (element
-// (m,k) at A + k*lda + m), as in the mma.sync GEMM of fvs_mlp.cu.
+// Operands are K-major (row m at A + m*lda) or MN-major (element (m,k) at A +
+// k*lda + m), as in the mma.sync GEMM of fvs_mlp.cu.  Leading dimensions and
+// the contiguous extents are multiples of 16 elements and the bases 16-byte
+// aligned (the padded layers of fvs_mlp.cu), so every 16-byte chunk lies
+// wholly inside or outside its matrix.
 //
-// CTA tile 128 x 128, K in blocks of 64 (four 128x128x16 MMAs), two shared
-// memory stages.  128 threads (one warpgroup):
-//   - all threads stage the operand tiles in the canonical K-major layout
-//     without swizzle (core matrices of 8 rows x 16 bytes): 16-byte vectors
-//     from K-major operands, element by element from transposed ones; then
-//     fence.proxy.async makes them visible to the tensor core;
+// CTA tile 128 x 64, K in blocks of 64 over two or four shared-memory stages
+// (48 or 96 KB).  256 threads (8 warps):
+//   - all threads bring the next blocks in with 16-byte cp.async, one or three
+//     blocks ahead, straight into the tensor core's canonical layouts without swizzle
+//     (core matrices of 8 rows x 16 bytes); chunks outside the matrix are
+//     zero-filled.  A warp's lanes run over the 8 rows of a core matrix first
+//     (no bank conflicts), then over 64 contiguous bytes of each row;
 //   - thread 0 issues the MMAs (tcgen05.mma.cta_group::1.kind::f16, M 128,
-//     N 128, K 16) and commits them to the stage's mbarrier, which frees the
-//     stage for the block two steps later;
-//   - after the last block, warp w reads accumulator rows 32w..32w+31
-//     (tensor-memory lanes) with tcgen05.ld, 32 columns at a time, transposes
-//     them through shared memory and writes whole row segments (coalesced)
-//     with the epilogue applied.
-// Split K (gridDim.z > 1): CTA z sums its own range of K blocks into the
-// partial matrix C + z * split_stride (raw accumulators, no epilogue);
-// k_sum_splits adds the partials in order (deterministic).
+//     N 64, K 16) and commits them to the stage's mbarrier, which frees it;
+//   - warp w reads the accumulator rows of tensor-memory lanes 32 (w % 4)..,
+//     32 columns from 32 (w / 4) (tcgen05.ld): a thread holds 32 consecutive
+//     columns of one row, applies the epilogue and stores 32-byte vectors.
+// The MLP's layers are 256 wide: with tiles of 128 x 128, two K stages filled
+// between barriers and one warpgroup, a 4096 x 256 x 256 layer ran on 64 CTAs
+// in 48 us, most of it waiting on loads and in the epilogue of 128 outputs a
+// thread; here it runs on 128 CTAs and 32 outputs a thread, in 10 us.
 // Every mbarrier wait is bounded (clock64 budget).  On expiry the kernel sets
 // *err, skips the remaining K blocks and the epilogue, waits for the MMAs it
 // already issued (bounded, up to 9 budgets in all), frees its tensor memory
@@ -35,33 +38,31 @@ namespace tc {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int BM = 128, BN = 128, BK = 64, THREADS = 128, STAGES = 2;
-constexpr int TILE_BYTES = BM * BK * 2;                  // one operand tile: 16 KB
-constexpr int SMEM_BYTES = STAGES * 2 * TILE_BYTES;      // 64 KB dynamic shared memory
-constexpr uint32_t TMEM_COLS = 128;                      // FP32 accumulator 128 x 128
-constexpr long long WAIT_BUDGET = 4000000000ll;          // clock cycles (~2 s at 2 GHz)
-
-// Byte offset of element (r, k) of a 128 x 64 tile: core matrices of 8 rows x
-// 8 elements stored as 128 contiguous bytes (row-major, 16 bytes a row); the
-// two core matrices of one 16-wide K step 128 bytes apart (leading byte
-// offset), 8-row groups 256 bytes apart (stride byte offset), K steps 4 KB apart.
-__host__ __device__ constexpr uint32_t tile_offset(int r, int k) {
-  return (uint32_t)((k >> 4) * 4096 + (r >> 3) * 256 + ((k >> 3) & 1) * 128 + (r & 7) * 16 + (k & 7) * 2);
-}
+constexpr int BM = 128, BN = 64, BK = 64, THREADS = 256;
+constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;  // one stage: 16 + 8 KB
+constexpr int smem_bytes(int stages) { return stages * (A_BYTES + B_BYTES); }
+constexpr uint32_t ACC_COLS = 64;                            // FP32 accumulator 128 x 64
+constexpr long long WAIT_BUDGET = 4000000000ll;              // clock cycles (~2 s at 2 GHz)
 
 // Shared-memory matrix descriptor: start address >> 4 (bits 0-13), leading
 // byte offset 128 >> 4 (bits 16-29), stride byte offset 256 >> 4 (bits 32-45),
 // descriptor version 1 (bits 46-47), base offset 0, no swizzle (bits 61-63 = 0).
+// In both canonical layouts used here (put_offset) the two core matrices of a
+// 16-wide K step are 128 bytes apart (leading offset) and the 8-element groups
+// along M or N 256 bytes apart (stride offset).
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
          ((uint64_t)1 << 46);
 }
 
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A BF16 (bits 7-9
-// = 1), B BF16 (bits 10-12 = 1), no negation, A and B K-major (bits 15, 16 =
-// 0), N >> 3 (bits 17-22), M >> 4 (bits 24-28).
-constexpr uint32_t IDESC =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+// = 1), B BF16 (bits 10-12 = 1), no negation, bit 15 / 16: A / B MN-major,
+// N >> 3 (bits 17-22), M >> 4 (bits 24-28).
+template <bool A_KM, bool B_KM>
+__host__ __device__ constexpr uint32_t idesc() {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (A_KM ? 0u : 1u << 15) | (B_KM ? 0u : 1u << 16) |
+         ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -81,75 +82,120 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
-template <bool KMAJOR>
-__device__ __forceinline__ void stage_tile(uint8_t* s, const bf16* g, int ld, int row0, int rows, int k0, int K) {
-  const int t = threadIdx.x;
-  if (KMAJOR) {
-    // 1024 chunks of 8 consecutive k (16 bytes), 8 per thread; 8 threads cover
-    // one 128-byte row segment (coalesced)
+// cp.async of 16 bytes; bytes = 0 fills with zeros and reads nothing
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// One operand's block of R rows (M or N) x 64 K into shared memory.  Chunk i
+// of 16 bytes: K-major, 8 consecutive k of row r; MN-major, 8 consecutive rows
+// of one k.  The place of a chunk: K steps of 16 R * 32 bytes apart, in a
+// step the groups of 8 rows 256 apart, the two groups of 8 k 128 apart, and
+// within a core matrix 16 bytes per row (K-major) or per k (MN-major).
+template <bool KMAJOR, int R>
+__device__ __forceinline__ void stage_block(uint32_t s, const bf16* g, int ld, int row0, int rows, int k0, int K) {
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const int i = q * THREADS + t;
-      const int r = i >> 3, kc = (i & 7) * 8;
-      const int gr = row0 + r, gk = k0 + kc;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (gr < rows) {
-        const bf16* src = g + (size_t)gr * ld + gk;
-        if (gk + 8 <= K && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0)) {
-          v = *reinterpret_cast<const uint4*>(src);
-        } else {
-          __align__(16) bf16 e[8];
-#pragma unroll
-          for (int j = 0; j < 8; j++) e[j] = gk + j < K ? src[j] : __float2bfloat16(0.f);
-          v = *reinterpret_cast<const uint4*>(e);
-        }
-      }
-      *reinterpret_cast<uint4*>(s + tile_offset(r, kc)) = v;
+  for (int q = 0; q < R * 8 / THREADS; q++) {
+    const int i = q * THREADS + (int)threadIdx.x;
+    const int lo = i & 7;
+    int r, k, off;
+    if (KMAJOR) {
+      // lanes: 8 rows, then 4 chunks along k; then the other 4 chunks, then the next 8 rows
+      const int c = (i >> 3) & 7;
+      r = ((i >> 6) << 3) + lo;
+      k = c << 3;
+      off = (c >> 1) * (R * 32) + (r >> 3) * 256 + (c & 1) * 128 + lo * 16;
+    } else {
+      // lanes: 8 k, then 4 chunks along the rows
+      const int c = (i >> 3) & (R / 8 - 1), kg = (i >> 3) / (R / 8);
+      r = c << 3;
+      k = (kg << 3) + lo;
+      off = (kg >> 1) * (R * 32) + c * 256 + (kg & 1) * 128 + lo * 16;
     }
-  } else {
-    // element (r, k) at g + k*ld + r: 8 consecutive r of one k per chunk
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const int i = q * THREADS + t;
-      const int k = i >> 4, rc = (i & 15) * 8;
-      const int gk = k0 + k, gr = row0 + rc;
-      __align__(16) bf16 e[8];
-#pragma unroll
-      for (int j = 0; j < 8; j++) e[j] = __float2bfloat16(0.f);
-      if (gk < K) {
-        const bf16* src = g + (size_t)gk * ld + gr;
-        if (gr + 8 <= rows && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0)) {
-          const uint4 v = *reinterpret_cast<const uint4*>(src);
-          *reinterpret_cast<uint4*>(e) = v;
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; j++)
-            if (gr + j < rows) e[j] = src[j];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 8; j++) *reinterpret_cast<bf16*>(s + tile_offset(rc + j, k)) = e[j];
-    }
+    const bool in = row0 + r < rows && k0 + k < K;
+    const bf16* src = KMAJOR ? g + (size_t)(row0 + r) * ld + (k0 + k) : g + (size_t)(k0 + k) * ld + (row0 + r);
+    cp_async16(s + off, in ? src : g, in ? 16u : 0u);
   }
 }
 
 __device__ __forceinline__ float gelu_tc(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
+__device__ __forceinline__ float gelu_grad_tc(float z) {
+  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
+}
 
-// epi: 0 = C only, 1 = C = acc + bias, 2 = C = acc + bias and Cact = GELU(C)
-template <bool A_KM, bool B_KM>
-__global__ void __launch_bounds__(THREADS) k_gemm_tc(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B,
-                                                     int ldb, int M, int N, int K, int epi,
-                                                     const float* __restrict__ bias, float* __restrict__ C, int ldc,
-                                                     bf16* __restrict__ Cact, int ldact, int* __restrict__ err,
-                                                     size_t split_stride) {
+// What becomes of the accumulator:
+//  OUT_RAW   C = acc (a split-K partial)
+//  OUT_PRED  C = acc + bias, the first nt columns only (ld nt)
+//  OUT_GELU  z = acc + bias; C = z (where C is given), H = BF16(GELU(z))
+//  OUT_MSE   z = acc + bias against the targets T[idx[m]][0..nt) (idx null: T[m]): H = BF16(2 (z - T) / (rows nt)),
+//            the squared errors added to *loss
+//  OUT_DGELU H = BF16(acc * GELU'(Z))
+enum Out : int { OUT_RAW = 0, OUT_PRED = 1, OUT_GELU = 2, OUT_MSE = 3, OUT_DGELU = 4 };
+
+struct GemmArgs {
+  const bf16* A;
+  const bf16* B;
+  int lda, ldb, M, N, K;
+  const float* bias;
+  float* C;        // ld N (rows of N columns)
+  bf16* H;         // ld N
+  const float* Z;  // ld N
+  const float* T;
+  const int* idx;
+  int nt;
+  float* loss;
+};
+
+// 32-byte accesses (a thread's columns are one row's, so a warp's access
+// touches 32 rows: the wider it is, the fewer passes it takes)
+__device__ __forceinline__ void ld8(const float* p, float* v) {
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "l"(p));
+}
+__device__ __forceinline__ void st8(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
+               "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
+// `ncol` (a multiple of 16, at most 32) of a thread's 32 columns; rows and
+// columns start at multiples of 32 bytes
+__device__ __forceinline__ void store_f32(float* p, const float* v, int ncol) {
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    if (8 * j < ncol) st8(p + 8 * j, v + 8 * j);
+}
+__device__ __forceinline__ void store_bf16(bf16* p, const float* v, int ncol) {
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+    if (16 * j < ncol) {
+      uint32_t h[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const __nv_bfloat162 q = __floats2bfloat162_rn(v[16 * j + 2 * i], v[16 * j + 2 * i + 1]);
+        h[i] = *reinterpret_cast<const uint32_t*>(&q);
+      }
+      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p + 16 * j), "r"(h[0]), "r"(h[1]), "r"(h[2]),
+                   "r"(h[3]), "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7])
+                   : "memory");
+    }
+}
+
+// One 128 x 64 output tile at (m0, n0) over the K blocks [kb0, kb0 + nk).
+// OUT_RAW sums each run of `per` blocks by itself: the accumulators of the
+// runs lie in two halves of the CTA's tensor memory in turn, so a run's partial
+// goes out (to C, C + run, ...) beside the next one's MMAs.
+template <bool A_KM, bool B_KM, int OUT, int STAGES>
+__device__ __forceinline__ void gemm_tile(const GemmArgs& a, int m0, int n0, int kb0, int nk, int per, size_t run,
+                                          int* err) {
+  constexpr uint32_t TMEM_COLS = OUT == OUT_RAW ? 2 * ACC_COLS : ACC_COLS;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t mbar[STAGES];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_ok;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  uint8_t* sA[STAGES] = {smem, smem + 2 * TILE_BYTES};
-  uint8_t* sB[STAGES] = {smem + TILE_BYTES, smem + 3 * TILE_BYTES};
+  const uint32_t sbase = smem_u32(smem);
 
   if (tid == 0) {
 #pragma unroll
@@ -168,45 +214,90 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(const bf16* __restrict__ A,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = tmem_slot;
+  // set up so far beside the tail of the kernel before; its results from here
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // K blocks of this CTA (all of them without split K)
-  const int nk_all = (K + BK - 1) / BK;
-  const int per = (nk_all + (int)gridDim.z - 1) / (int)gridDim.z;
-  const int kb0 = (int)blockIdx.z * per;
-  const int nk = max(0, min(nk_all - kb0, per));
-  if (gridDim.z > 1) C += (size_t)blockIdx.z * split_stride;
+  auto load = [&](int kb) {  // one commit group per call, empty past the last block
+    if (kb < nk) {
+      const uint32_t s = sbase + (uint32_t)(kb % STAGES) * (A_BYTES + B_BYTES);
+      stage_block<A_KM, BM>(s, a.A, a.lda, m0, a.M, (kb0 + kb) * BK, a.K);
+      stage_block<B_KM, BN>(s + A_BYTES, a.B, a.ldb, n0, a.N, (kb0 + kb) * BK, a.K);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+#pragma unroll
+  for (int kb = 0; kb < STAGES - 1; kb++) load(kb);
+  // the accumulator of this warp's 32 rows and 32 columns
+  const int c0 = (warp >> 2) * 32;
+  auto read_acc = [&](uint32_t acc, uint32_t* u) {
+    const uint32_t taddr = acc + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+          "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]),
+          "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]),
+          "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+  };
+  const int m = m0 + (warp & 3) * 32 + lane, n = n0 + c0;
+  const int ncol = min(32, a.N - n);  // a multiple of 16; <= 0: columns past the matrix
+  // the partial of run r, once its MMAs are complete
+  auto store_run = [&](int r) {
+    uint32_t u[32];
+    read_acc(tmem + (uint32_t)(r & 1) * ACC_COLS, u);
+    if (m < a.M && ncol > 0)
+      store_f32(a.C + (size_t)r * run + (size_t)m * a.N + n, reinterpret_cast<const float*>(u), ncol);
+  };
   int issued = -1;  // last K block whose MMAs thread 0 committed
   for (int kb = 0; kb < nk; kb++) {
-    const int s = kb & 1;
-    if (kb >= STAGES) {
-      // the MMAs of block kb-2 read this stage: wait for their commit
-      if (tid == 0 && !mbar_wait(smem_u32(&mbar[s]), (uint32_t)(((kb - STAGES) >> 1) & 1))) s_ok = 0;
-      __syncthreads();
-      if (!s_ok) break;
-    }
-    stage_tile<A_KM>(sA[s], A, lda, m0, M, (kb0 + kb) * BK, K);
-    stage_tile<B_KM>(sB[s], B, ldb, n0, N, (kb0 + kb) * BK, K);
+    // block kb has arrived (all but the newest STAGES - 2 groups)
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const uint32_t a0 = smem_u32(sA[s]), b0 = smem_u32(sB[s]);
-#pragma unroll
-      for (int kk = 0; kk < BK / 16; kk++) {
-        const uint64_t ad = smem_desc(a0 + kk * 4096), bd = smem_desc(b0 + kk * 4096);
-        const uint32_t acc = (kb > 0 || kk > 0) ? 1u : 0u;
+      const uint32_t a0 = sbase + (uint32_t)(kb % STAGES) * (A_BYTES + B_BYTES), b0 = a0 + A_BYTES;
+      const int steps = min(BK / 16, (a.K - (kb0 + kb) * BK + 15) / 16);
+      for (int kk = 0; kk < steps; kk++) {
+        const uint64_t ad = smem_desc(a0 + kk * (BM * 32)), bd = smem_desc(b0 + kk * (BN * 32));
+        const uint32_t acc = ((OUT == OUT_RAW ? kb % per > 0 : kb > 0) || kk > 0) ? 1u : 0u;
+        const uint32_t dst = OUT == OUT_RAW ? tmem + (uint32_t)((kb / per) & 1) * ACC_COLS : tmem;
         asm volatile(
             "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-            "l"(ad), "l"(bd), "r"(IDESC), "r"(acc)
+            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dst),
+            "l"(ad), "l"(bd), "r"(idesc<A_KM, B_KM>()), "r"(acc)
             : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                       smem_u32(&mbar[s]))
+                       smem_u32(&mbar[kb % STAGES]))
                    : "memory");
       issued = kb;
     }
+    // block kb + STAGES - 1 goes where block kb - 1 was: wait for that block's MMAs;
+    // a run's partial goes out after the next run's first block was issued
+    const bool run_done = OUT == OUT_RAW && kb > 0 && kb % per == 0;
+    if ((kb + STAGES - 1 < nk || run_done) && kb > 0) {
+      if (tid == 0 && !mbar_wait(smem_u32(&mbar[(kb - 1) % STAGES]), (uint32_t)(((kb - 1) / STAGES) & 1))) s_ok = 0;
+      __syncthreads();
+      if (!s_ok) break;
+    }
+    load(kb + STAGES - 1);
+    if (OUT == OUT_RAW && run_done) {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      store_run(kb / per - 1);
+      // (the accumulator is written again one run later, after further block barriers)
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    }
   }
+  // the successor may be scheduled beside the epilogue (it waits for this
+  // grid's results)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // No copy may land in shared memory after the CTA has exited (an early
+  // break leaves groups in flight)
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   // Every MMA this CTA issued must be complete before its tensor memory is
   // read or freed, and before the CTA exits (the MMAs read the operand
   // stages in shared memory).  The commit of the last issued block tracks
@@ -214,11 +305,11 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(const bf16* __restrict__ A,
   // wait also runs after an earlier wait ran out (s_ok == 0, loop left
   // early).  The MMAs' operands are staged and nothing else gates them, so
   // the tensor core completes them; only a GPU stalled for the whole budget
-  // makes the wait expire.  Then it is repeated once with 8 times the
-  // budget, and the CTA frees its tensor memory only after that: freeing it
-  // earlier could let a later CTA's accumulator receive these MMAs' writes.
+  // makes the wait expire.  Then it is repeated with 8 times the budget, and
+  // the CTA frees its tensor memory only after that: freeing it earlier could
+  // let a later CTA's accumulator receive these MMAs' writes.
   if (tid == 0 && issued >= 0) {
-    const uint32_t fb = smem_u32(&mbar[issued & 1]), fp = (uint32_t)((issued >> 1) & 1);
+    const uint32_t fb = smem_u32(&mbar[issued % STAGES]), fp = (uint32_t)((issued / STAGES) & 1);
     if (!mbar_wait(fb, fp)) {
       s_ok = 0;
       for (int r = 0; r < 8 && !mbar_wait(fb, fp); r++) {
@@ -227,44 +318,60 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(const bf16* __restrict__ A,
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  if (s_ok) {
-    // transpose staging, one 32 x 33 float tile per warp, in the (now free)
-    // operand stages
-    float* st = reinterpret_cast<float*>(smem) + warp * (32 * 33);
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
-      uint32_t v[32];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-          "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-            "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-            "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-            "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-          : "r"(taddr)
-          : "memory");
-      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-      // lane = row: v[j] is column c0 + j; write the tile, read it back by
-      // column so that each store instruction covers 32 consecutive columns
-      if (nk == 0) {
+  if (s_ok && OUT == OUT_RAW) {
+    if (nk > 0) store_run((nk - 1) / per);
+  } else if (s_ok) {
+    uint32_t u[32];
+    read_acc(tmem, u);
+    float v[32], e2 = 0.f;
 #pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = 0u;  // an empty K range contributes zeros
-      }
+    for (int j = 0; j < 32; j++) v[j] = __uint_as_float(u[j]);
+    if (m < a.M && ncol > 0) {
+      const size_t at = (size_t)m * a.N + n;
+      if (OUT == OUT_PRED || OUT == OUT_GELU || OUT == OUT_MSE) {
 #pragma unroll
-      for (int j = 0; j < 32; j++) st[lane * 33 + j] = __uint_as_float(v[j]);
-      __syncwarp();
-      const int n = n0 + c0 + lane;
-      const float bn = (epi != 0 && bias && n < N) ? bias[n] : 0.f;
-#pragma unroll 4
-      for (int r = 0; r < 32; r++) {
-        const int m = m0 + warp * 32 + r;
-        if (m >= M || n >= N) continue;
-        const float z = st[r * 33 + lane] + bn;
-        if (C) C[(size_t)m * ldc + n] = z;
-        if (epi == 2 && Cact) Cact[(size_t)m * ldact + n] = __float2bfloat16(gelu_tc(z));
+        for (int j = 0; j < 32; j++)
+          if (j < ncol) v[j] += a.bias[n + j];
       }
-      __syncwarp();
+      if (OUT == OUT_GELU && a.C) store_f32(a.C + at, v, ncol);
+      if (OUT == OUT_PRED) {
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+          if (n + j < a.nt) a.C[(size_t)m * a.nt + n + j] = v[j];
+      }
+      if (OUT == OUT_GELU) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = gelu_tc(v[j]);
+        store_bf16(a.H + at, v, ncol);
+      }
+      if (OUT == OUT_MSE) {
+        const float* t = a.T + (size_t)(a.idx ? a.idx[m] : m) * a.nt;
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+          float d = 0.f;
+          if (n + j < a.nt) {
+            d = v[j] - t[n + j];
+            e2 += d * d;
+          }
+          v[j] = 2.f * d / float(a.M * a.nt);
+        }
+        store_bf16(a.H + at, v, ncol);
+      }
+      if (OUT == OUT_DGELU) {
+        float z[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++) z[j] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (8 * j < ncol) ld8(a.Z + at + 8 * j, z + 8 * j);
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = v[j] * gelu_grad_tc(z[j]);
+        store_bf16(a.H + at, v, ncol);
+      }
+    }
+    if (OUT == OUT_MSE) {
+      for (int o = 16; o > 0; o >>= 1) e2 += __shfl_down_sync(0xffffffffu, e2, o);
+      if (lane == 0 && e2 != 0.f) atomicAdd(a.loss, e2);
     }
   } else if (tid == 0) {
     atomicExch(err, 1);
@@ -276,17 +383,119 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(const bf16* __restrict__ A,
   }
 }
 
-// C[m][n] = sum over z of the split partials P[z][m][n] (ldc, stride), in
-// order z = 0, 1, ... (deterministic)
-__global__ void k_sum_splits(const float* __restrict__ P, int nsplit, size_t stride, int M, int N, int ldc,
-                             float* __restrict__ C) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= (size_t)M * N) return;
-  const int m = (int)(i / N), n = (int)(i % N);
-  const size_t o = (size_t)m * ldc + n;
-  float acc = 0.f;
-  for (int z = 0; z < nsplit; z++) acc += P[z * stride + o];
-  C[o] = acc;
+// one GEMM: a CTA per 128 x 64 tile (x along N)
+template <bool A_KM, bool B_KM, int OUT, int STAGES>
+__global__ void __launch_bounds__(THREADS, STAGES == 2 ? (OUT == OUT_DGELU ? 3 : 4) : 2) k_gemm_tc(const GemmArgs a, int* __restrict__ err) {
+  gemm_tile<A_KM, B_KM, OUT, STAGES>(a, (int)blockIdx.y * BM, (int)blockIdx.x * BN, 0, (a.K + BK - 1) / BK, 1, 0, err);
+}
+
+// All weight gradients of a network, dW_l[n][k] = sum_m dZ_l[m][n] X_l[m][k],
+// and bias gradients, db_l[n] = sum_m dZ_l[m][n], in one launch.  K is the
+// batch: a layer's K blocks are summed in runs of `per`, and the runs' partial
+// sums added in order by k_finish_grads (deterministic).  A CTA takes `runs`
+// consecutive runs of one 128 x 64 tile; a bias CTA 32 columns of one layer's
+// dZ, each column in 32 interleaved row sums added in order.
+constexpr int MAX_LAYERS = 17, BIAS_COLS = 32;
+struct GradLayer {
+  const bf16* dZ;  // [rows][dout]
+  const bf16* X;   // [rows][din]
+  int din, dout;
+  int tiles_n, tiles;  // tiles along din, and in all
+  int per, nsplit;     // K blocks of a run, runs
+  int cta0, bias0;     // first CTA of the layer's tiles, and of its bias columns
+  size_t part;         // offset of its partial sums: [nsplit][dout][din], then db[dout]
+  size_t w0, b0;       // its weights and biases in the parameter vector
+};
+struct GradPlan {
+  int nl, rows, runs;
+  int gemm_ctas, ctas;
+  GradLayer l[MAX_LAYERS];
+};
+
+__global__ void __launch_bounds__(THREADS, 4) k_grads(const GradPlan p, float* __restrict__ part, int* __restrict__ err) {
+  const int b = (int)blockIdx.x;
+  if (b < p.gemm_ctas) {
+    int l = 0;
+    while (l + 1 < p.nl && b >= p.l[l + 1].cta0) l++;
+    const GradLayer& g = p.l[l];
+    const int i = b - g.cta0, tile = i % g.tiles, z = i / g.tiles * p.runs;
+    GemmArgs a = {};
+    a.A = g.dZ; a.lda = g.dout; a.M = g.dout;
+    a.B = g.X; a.ldb = g.din; a.N = g.din;
+    a.K = p.rows;
+    const size_t run = (size_t)g.dout * g.din;
+    a.C = part + g.part + (size_t)z * run;
+    const int nk = (p.rows + BK - 1) / BK, kb0 = z * g.per;
+    gemm_tile<false, false, OUT_RAW, 2>(a, tile / g.tiles_n * BM, tile % g.tiles_n * BN, kb0,
+                                     max(0, min(nk - kb0, p.runs * g.per)), g.per, run, err);
+    return;
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int l = 0;
+  while (l + 1 < p.nl && b >= p.l[l + 1].bias0) l++;
+  const GradLayer& g = p.l[l];
+  extern __shared__ __align__(128) uint8_t smem[];
+  float(*sh)[BIAS_COLS] = reinterpret_cast<float(*)[BIAS_COLS]>(smem);  // [32][32]
+  const int col0 = (b - g.bias0) * BIAS_COLS, c = col0 + 4 * ((int)threadIdx.x & 7), ty = (int)threadIdx.x >> 3;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  if (c < g.dout) {
+#pragma unroll 16
+    for (int r = ty; r < p.rows; r += 32) {
+      const uint2 q = *reinterpret_cast<const uint2*>(g.dZ + (size_t)r * g.dout + c);
+      const bf16* h = reinterpret_cast<const bf16*>(&q);
+#pragma unroll
+      for (int j = 0; j < 4; j++) s[j] += __bfloat162float(h[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++) sh[ty][c - col0 + j] = s[j];
+  __syncthreads();
+  const int o = col0 + (int)threadIdx.x;
+  if (threadIdx.x < BIAS_COLS && o < g.dout) {
+    float t = 0.f;
+    for (int q = 0; q < 32; q++) t += sh[q][threadIdx.x];
+    part[g.part + (size_t)g.nsplit * g.dout * g.din + o] = t;
+  }
+}
+
+// Adam's constants of a step (bc1, bc2: bias corrections 1 - beta^step)
+struct AdamArgs {
+  float lr, b1, b2, eps, bc1, bc2;
+};
+
+// Gradient of every parameter from its partial sums, added in order; with
+// ADAM also the update of the moments, the FP32 parameters and their BF16 copy.
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_finish_grads(const GradPlan p, const float* __restrict__ part, size_t n,
+                                                      float* __restrict__ grad, float* __restrict__ w,
+                                                      float* __restrict__ am, float* __restrict__ av,
+                                                      bf16* __restrict__ wb, AdamArgs ad) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int l = 0;
+  while (l + 1 < p.nl && i >= p.l[l + 1].w0) l++;
+  const GradLayer& g = p.l[l];
+  const size_t nw = (size_t)g.dout * g.din;
+  float gi = 0.f;
+  if (i < g.b0) {
+    const float* s = part + g.part + (i - g.w0);
+#pragma unroll 16
+    for (int z = 0; z < g.nsplit; z++) gi += s[z * nw];
+  } else {
+    gi = part[g.part + (size_t)g.nsplit * nw + (i - g.b0)];
+  }
+  if (!ADAM) {
+    grad[i] = gi;
+    return;
+  }
+  const float mi = ad.b1 * am[i] + (1.f - ad.b1) * gi;
+  const float vi = ad.b2 * av[i] + (1.f - ad.b2) * gi * gi;
+  am[i] = mi;
+  av[i] = vi;
+  const float wi = w[i] - ad.lr * (mi / ad.bc1) / (sqrtf(vi / ad.bc2) + ad.eps);
+  w[i] = wi;
+  wb[i] = __float2bfloat16(wi);
 }
 
 }  // namespace tc
