@@ -56,7 +56,11 @@ __host__ __device__ __forceinline__ df64 two_sum(float a, float b) {
   return df64(s, (a - (s - bp)) + (b - bp));
 }
 __host__ __device__ __forceinline__ df64 two_prod(float a, float b) {
+#ifdef __CUDA_ARCH__
+  const float p = __fmul_rn(a, b);  // not to be contracted into a sum that takes p
+#else
   const float p = a * b;
+#endif
   return df64(p, fmaf(a, b, -p));
 }
 
@@ -93,6 +97,23 @@ __device__ __forceinline__ df64 dsqrt_(df64 x) {
   const df64 p = two_prod(s, s);
   const float r = ((x.hi - p.hi) - p.lo) + x.lo;
   return fast_two_sum(s, __fdiv_rn(r, 2.0f * s));
+}
+// 1 / x and 1 / sqrt(x) of positive normal numbers: the FP32 approximation y
+// corrected by its residual e, formed in one or two exact products: y (1 + e +
+// e^2) with e = 1 - x y, and y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2 (the
+// series forms of fp64_fast.cuh).  |e| < 2^-21, so what is left out lies below
+// 2^-63 and the correction, rounded to FP32, is exact to 2^-45 of the result or better.
+__device__ __forceinline__ df64 drcp_(df64 x) {
+  const float y = __frcp_rn(x.hi);
+  const float e = __fmaf_rn(-x.lo, y, __fmaf_rn(-x.hi, y, 1.0f));
+  return fast_two_sum(y, y * __fmaf_rn(e, e, e));
+}
+__device__ __forceinline__ df64 drsqrt_(df64 x) {
+  const float y = rsqrtf(x.hi);
+  const df64 p = two_prod(y, y);
+  const df64 q = two_prod(x.hi, p.hi);  // q + the terms below: x y^2
+  const float e = (1.0f - q.hi) - (q.lo + __fmaf_rn(x.hi, p.lo, x.lo * p.hi));
+  return fast_two_sum(y, y * e * __fmaf_rn(0.375f, e, 0.5f));
 }
 // a + b, sloppy: one TwoSum of the high parts, the low parts added to its
 // error, renormalised

@@ -218,7 +218,7 @@ void init_view_constants(fvs_batch* B, DevView& d) {
   d.gamma = ob.gamma; d.gm1 = ob.gamma - 1.0; d.igm1 = 1.0 / (ob.gamma - 1.0);
   d.ggm1 = ob.gamma / (ob.gamma - 1.0);
   d.khalf = ob.umuscl / 2.0; d.nkhalf = -ob.umuscl / 2.0; d.omk = 1.0 - ob.umuscl; d.cfl = ob.cfl;
-  set_fp32_constants(d);
+  set_constants(d);
   d.limiter = ob.limiter; d.grad_method = ob.grad_method; d.first_order = ob.reconst == FVS_RECON_UPWIND1;
   d.vortex = ob.vortex; d.vx = ob.vortex_x; d.vy = ob.vortex_y; d.vkappa = ob.vortex_kappa;
   for (int k = 0; k < 4; k++) { d.vinf[k] = ob.vortex_inf[k]; d.pinf[k] = B->pinf[k]; }
@@ -994,7 +994,7 @@ int fvs_batch_run_to_level_dc(fvs_batch* b, int32_t max_steps, const double* lev
     // base state of the chunk: fold, FP64 residual and wave speeds, FP32 copies
     K.fold(*d32, b->dc, d64.U, b->stream);
     K64.cvar2pvar(d64, b->stream);
-    K64.flux(d64, 0.0, true, b->stream);
+    K64.flux_base(d64, b->stream);
     K64.residual_out(d64, b->stream);
     K.base(*d32, b->dc, d64.U, d64.resid, d64.ws, b->stream);
     *b->h_step0 = step;

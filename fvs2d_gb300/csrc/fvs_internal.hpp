@@ -124,6 +124,7 @@ struct DevView {
   const int2* ecell = nullptr;    // (L,R) device cell ids; R = -1 on boundary edges
   const void* enrm = nullptr;     // [nedge] x 2 unit normal (T)
   const void* earea = nullptr;    // [nedge] (T)
+  const double* efac = nullptr;   // [nedge] x 4: length / 2 times (nx, ny, 1, 1/2) (FP64 build's flux)
   const void* edL = nullptr;      // [nedge] x 2 xf - xcL (T)
   const void* edR = nullptr;      // [nint] x 2 xf - xcR (T)
   const int* ebtype = nullptr;    // [nedge] boundary record: type | case << 4 (boundary slots only)
@@ -144,6 +145,7 @@ struct DevView {
   // scheme
   double gamma = 1.4, khalf = 0, nkhalf = 0, omk = 1, cfl = 1, dt = 0;
   double gm1 = 0.4, igm1 = 2.5, ggm1 = 3.5;  // gamma-1, 1/(gamma-1) and gamma/(gamma-1)
+  double hgm1 = 0.2, c2 = 7.0;               // (gamma-1)/2 and 2 gamma/(gamma-1)
   // the same constants rounded once on the host for the FP32 kernels
   float fgamma = 1.4f, fgm1 = 0.4f, figm1 = 2.5f, fkhalf = 0, fnkhalf = 0, fomk = 1, fggm1 = 3.5f;
   // and split into FP32 pairs (hi, lo) for the double-float kernels
@@ -156,8 +158,11 @@ struct DevView {
   double mc[16];
 };
 
-// FP32 constants of the scheme: rounded, and split into (hi, lo) pairs
-inline void set_fp32_constants(DevView& d) {
+// constants derived from the scheme's: exact multiples, rounded to FP32, and
+// split into (hi, lo) pairs
+inline void set_constants(DevView& d) {
+  d.hgm1 = 0.5 * d.gm1;
+  d.c2 = 2.0 * d.ggm1;
   auto split = [](double x, float* o) {
     o[0] = float(x);
     o[1] = float(x - double(o[0]));
@@ -318,6 +323,8 @@ struct KernelSet {
   // blocks of 256 threads of the update kernel of an RK mode resident on the
   // device at once (0: unknown); queried before any graph capture
   int (*update_wave)(int mode);
+  // first-order flux of a defect-correction chunk's base state (FP64 build)
+  void (*flux_base)(const DevView&, cudaStream_t) = nullptr;
 };
 // Defect correction of a first-order steady batch (mixed build): per chunk
 // the FP64 residual R0 of the base state is evaluated once; the RK stages

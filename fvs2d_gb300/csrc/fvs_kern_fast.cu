@@ -11,7 +11,7 @@ const KernelSet& kernels_fp64_fast() {
                               k_fast::launch_flux, k_fast::launch_update, k_fast::launch_residual_out, k_fast::persistent_occupancy,
                               k_fast::launch_persistent, k_fast::launch_tiled_step,
                               nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                              k_fast::update_wave};
+                              k_fast::update_wave, k_fast::launch_flux_base};
   return k;
 }
 }  // namespace fvs
