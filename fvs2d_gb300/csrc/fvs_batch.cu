@@ -796,7 +796,9 @@ int fvs_batch_steps(fvs_batch* b, int32_t nsteps, double* norms, float* ms) {
 int fvs_batch_autotune(fvs_batch* b, int32_t trial_steps, float* best_ms) {
   NvtxRange nv("fvs batch autotune");
   if (!b || trial_steps <= 0 || trial_steps > b->norm_cap) return FVS_ERR_INVALID;
-  cudaError_t e = cudaMemcpy(b->d_backup, b->d.U, 32 * (size_t)b->nc, cudaMemcpyDeviceToDevice);
+  // (on the batch's stream: a device-to-device cudaMemcpy on the legacy stream
+  // neither waits for that stream nor holds up the host)
+  cudaError_t e = cudaMemcpyAsync(b->d_backup, b->d.U, 32 * (size_t)b->nc, cudaMemcpyDeviceToDevice, b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "state backup");
   const int blocks[2] = {128, 256};
   const int tiles_per_block[3] = {1, 4, 16};
@@ -839,7 +841,7 @@ int fvs_batch_autotune(fvs_batch* b, int32_t trial_steps, float* best_ms) {
   b->tiled = btiled;
   b->fuse = bfuse;
   b->plan_dirty = true;
-  e = cudaMemcpy(b->d.U, b->d_backup, 32 * (size_t)b->nc, cudaMemcpyDeviceToDevice);
+  e = cudaMemcpyAsync(b->d.U, b->d_backup, 32 * (size_t)b->nc, cudaMemcpyDeviceToDevice, b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "state restore");
   // primitives of the restored state
   b->ks->cvar2pvar(b->d, b->stream);

@@ -629,8 +629,8 @@ static int copy_params(fvs_mlp* m, float* host, const float* in, int64_t n, bool
   if (!get) {
     if (cudaMemcpy(m->w, pad.data(), 4 * m->nparam, cudaMemcpyHostToDevice) != cudaSuccess)
       return m->fail(FVS_ERR_CUDA, "parameter upload");
-    cudaMemset(m->am, 0, 4 * m->nparam);
-    cudaMemset(m->av, 0, 4 * m->nparam);
+    cudaMemsetAsync(m->am, 0, 4 * m->nparam, m->stream);
+    cudaMemsetAsync(m->av, 0, 4 * m->nparam, m->stream);
     m->step = 0;
     refresh_bf16(m);
     return check(m, "set_params");
