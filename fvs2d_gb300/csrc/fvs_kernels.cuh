@@ -1264,6 +1264,27 @@ __global__ void __launch_bounds__(256) k_flux(const DevView d, double dts, int w
 // ---------------------------------------------------------------------------
 // per-cell gather of the edge slots in the reference's summation order
 // ---------------------------------------------------------------------------
+// What the gather of a cell reads that no kernel of a step writes: its slots
+// and -1/vol (the strict build: vol)
+struct CellStatic {
+  int4 cf;
+#if FVS_MIXED || FVS_DF
+  T rv;
+#else
+  double rv;
+#endif
+  __device__ __forceinline__ void load(const DevView& d, int ic) {
+    cf = d.cflist[ic];
+#if FVS_MIXED || FVS_DF
+    rv = -static_cast<const T*>(d.volT)[ic];
+#elif FVS_STRICT
+    rv = d.vol[ic];
+#else
+    rv = -d.rvol[ic];
+#endif
+  }
+};
+
 #if FVS_MIXED
 // FP32 flux slots summed with an error-free transformation (TwoSum): hi + lo
 // equals the exact sum of the slots to ~2^-48 relative, then one FP64 add per
@@ -1322,11 +1343,9 @@ __device__ __forceinline__ void residual_from_faces_df(const int* sl, df64 rv, G
 }
 
 template <bool WS, bool COH>
-__device__ __forceinline__ void cell_residual_df(const DevView& d, int ic, df64* res, double& ws) {
-  const int4 cf = d.cflist[ic];
-  const int sl[4] = {cf.x, cf.y, cf.z, cf.w};
-  const df64 rv = -static_cast<const df64*>(d.volT)[ic];
-  residual_from_faces_df<WS>(sl, rv, [&](int idx, df64* f, df64& w) {
+__device__ __forceinline__ void cell_residual_df(const DevView& d, const CellStatic& c, df64* res, double& ws) {
+  const int sl[4] = {c.cf.x, c.cf.y, c.cf.z, c.cf.w};
+  residual_from_faces_df<WS>(sl, c.rv, [&](int idx, df64* f, df64& w) {
     ldc4<COH>(static_cast<const df64*>(d.eflux), idx, f);
     if (WS) w = ldc1<COH>(static_cast<const df64*>(d.ews), idx);
   }, res, ws);
@@ -1336,7 +1355,9 @@ __device__ __forceinline__ void cell_residual_df(const DevView& d, int ic, df64*
 template <bool WS, bool COH>
 __device__ __forceinline__ void cell_residual(const DevView& d, int ic, double* res, double& ws) {
   df64 r[4];
-  cell_residual_df<WS, COH>(d, ic, r, ws);
+  CellStatic c;
+  c.load(d, ic);
+  cell_residual_df<WS, COH>(d, c, r, ws);
 #pragma unroll
   for (int v = 0; v < 4; v++) res[v] = to_double(r[v]);
 }
@@ -1361,9 +1382,8 @@ __device__ __forceinline__ void gather_slot(const DevView& d, int s, double* r, 
 // order); the FP64 build starts the sums from the first slot instead of from
 // zero (the same values, four additions fewer)
 template <bool WS, bool COH>
-__device__ __forceinline__ void cell_flux_sum(const DevView& d, int ic, double* r, double& ws) {
+__device__ __forceinline__ void cell_flux_sum(const DevView& d, int4 cf, double* r, double& ws) {
   ws = 0.0;
-  const int4 cf = d.cflist[ic];
 #if FVS_STRICT
 #pragma unroll
   for (int v = 0; v < 4; v++) r[v] = 0.0;
@@ -1388,18 +1408,22 @@ __device__ __forceinline__ void cell_flux_sum(const DevView& d, int ic, double* 
 }
 
 template <bool WS, bool COH>
-__device__ __forceinline__ void cell_residual(const DevView& d, int ic, double* res, double& ws) {
+__device__ __forceinline__ void cell_residual(const DevView& d, const CellStatic& c, double* res, double& ws) {
   double r[4];
-  cell_flux_sum<WS, COH>(d, ic, r, ws);
+  cell_flux_sum<WS, COH>(d, c.cf, r, ws);
+#pragma unroll
 #if FVS_STRICT
-  const double vol = d.vol[ic];
-#pragma unroll
-  for (int v = 0; v < 4; v++) res[v] = -r[v] / vol;  // src/residual.f90:164-166
+  for (int v = 0; v < 4; v++) res[v] = -r[v] / c.rv;  // src/residual.f90:164-166
 #else
-  const double rv = -d.rvol[ic];
-#pragma unroll
-  for (int v = 0; v < 4; v++) res[v] = r[v] * rv;
+  for (int v = 0; v < 4; v++) res[v] = r[v] * c.rv;
 #endif
+}
+
+template <bool WS, bool COH>
+__device__ __forceinline__ void cell_residual(const DevView& d, int ic, double* res, double& ws) {
+  CellStatic c;
+  c.load(d, ic);
+  cell_residual<WS, COH>(d, c, res, ws);
 }
 #endif
 
@@ -1567,11 +1591,10 @@ __device__ __forceinline__ void residual_from_faces_f(const int* sl, float rv, b
   ws = wh + wl;
 }
 
-__device__ __forceinline__ void cell_residual_f(const DevView& d, int ic, bool want_ws, float* res, float& ws) {
-  const int4 cf = d.cflist[ic];
-  const int sl[4] = {cf.x, cf.y, cf.z, cf.w};
-  const float rv = -static_cast<const float*>(d.volT)[ic];
-  residual_from_faces_f(sl, rv, want_ws, [&](int idx, float* f, float& w) {
+__device__ __forceinline__ void cell_residual_f(const DevView& d, const CellStatic& c, bool want_ws, float* res,
+                                                float& ws) {
+  const int sl[4] = {c.cf.x, c.cf.y, c.cf.z, c.cf.w};
+  residual_from_faces_f(sl, c.rv, want_ws, [&](int idx, float* f, float& w) {
     ldc4<true>(static_cast<const float*>(d.eflux), idx, f);
     if (want_ws) w = ldc1<true>(static_cast<const float*>(d.ews), idx);
   }, res, ws);
@@ -1665,9 +1688,10 @@ __device__ __forceinline__ void apply_stage_f(const DevView& d, const StageParam
 }
 
 template <int MODE, bool COH>
-__device__ __forceinline__ void update_item(const DevView& d, const StageParams& sp, int ic, NormAcc& na) {
+__device__ __forceinline__ void update_item(const DevView& d, const StageParams& sp, int ic, const CellStatic& c,
+                                            NormAcc& na) {
   float res[4], ws;
-  cell_residual_f(d, ic, sp.steady && sp.stage == 1, res, ws);
+  cell_residual_f(d, c, sp.steady && sp.stage == 1, res, ws);
   apply_stage_f<MODE, COH>(d, sp, ic, res, ws, static_cast<float*>(d.Pv), na);
 }
 
@@ -1843,31 +1867,40 @@ __device__ __forceinline__ void apply_stage_df(const DevView& d, const StagePara
 
 // one cell of an RK stage; at the last stage adds |U-U0|^2 to na
 template <int MODE, bool COH>
-__device__ __forceinline__ void update_item(const DevView& d, const StageParams& sp, int ic, NormAcc& na) {
+__device__ __forceinline__ void update_item(const DevView& d, const StageParams& sp, int ic, const CellStatic& c,
+                                            NormAcc& na) {
   df64 res[4];
   double ws;
-  if (sp.steady && sp.stage == 1) cell_residual_df<true, COH>(d, ic, res, ws);
-  else cell_residual_df<false, COH>(d, ic, res, ws);
+  if (sp.steady && sp.stage == 1) cell_residual_df<true, COH>(d, c, res, ws);
+  else cell_residual_df<false, COH>(d, c, res, ws);
   apply_stage_df<MODE, COH>(d, sp, ic, res, ws, static_cast<T*>(d.Pv), na);
 }
 #else
 // one cell of an RK stage; at the last stage adds |U-U0|^2 to na
 template <int MODE, bool COH>
-__device__ __forceinline__ void update_item(const DevView& d, const StageParams& sp, int ic, NormAcc& na) {
+__device__ __forceinline__ void update_item(const DevView& d, const StageParams& sp, int ic, const CellStatic& c,
+                                            NormAcc& na) {
   double res[4], ws;
 #if FVS_STRICT
-  if (sp.steady && sp.stage == 1) cell_residual<true, COH>(d, ic, res, ws);
-  else cell_residual<false, COH>(d, ic, res, ws);
+  if (sp.steady && sp.stage == 1) cell_residual<true, COH>(d, c, res, ws);
+  else cell_residual<false, COH>(d, c, res, ws);
   apply_stage_d<MODE, COH>(d, sp, ic, res, ws, static_cast<T*>(d.Pv), na);
 #else
-  if (sp.steady && sp.stage == 1) cell_flux_sum<true, COH>(d, ic, res, ws);
-  else cell_flux_sum<false, COH>(d, ic, res, ws);
-  apply_stage_d<MODE, COH, true>(d, sp, ic, res, ws, static_cast<T*>(d.Pv), na, -d.rvol[ic]);
+  if (sp.steady && sp.stage == 1) cell_flux_sum<true, COH>(d, c.cf, res, ws);
+  else cell_flux_sum<false, COH>(d, c.cf, res, ws);
+  apply_stage_d<MODE, COH, true>(d, sp, ic, res, ws, static_cast<T*>(d.Pv), na, c.rv);
 #endif
 }
 #endif
 
 #endif  // FVS_MIXED
+
+template <int MODE, bool COH>
+__device__ __forceinline__ void update_item(const DevView& d, const StageParams& sp, int ic, NormAcc& na) {
+  CellStatic c;
+  c.load(d, ic);
+  update_item<MODE, COH>(d, sp, ic, c, na);
+}
 
 // RMS of |U - U0| per component from the block partials, by one block in a
 // fixed order (deterministic); advances the step counter.  sh: the shared
@@ -1939,15 +1972,23 @@ __device__ __forceinline__ void stage_norms(const DevView& d, NormAcc& na, void*
 // stage's launch); otherwise one cell per thread.
 template <int MODE, bool STRIDE>
 __global__ void __launch_bounds__(256) k_update(const DevView d, const StageParams sp) {
+  int ic = blockIdx.x * blockDim.x + threadIdx.x;
+  CellStatic c;
+  if (ic < d.nc) c.load(d, ic);
   pdl_wait();
   if (d.trig_first) pdl_trigger();
   NormAcc na;
   if (STRIDE) {
-    for (int ic = blockIdx.x * blockDim.x + threadIdx.x; ic < d.nc; ic += gridDim.x * blockDim.x)
-      update_item<MODE, false>(d, sp, ic, na);
+    while (ic < d.nc) {
+      const int next = ic + gridDim.x * blockDim.x;
+      CellStatic cn;
+      if (next < d.nc) cn.load(d, next);
+      update_item<MODE, false>(d, sp, ic, c, na);
+      c = cn;
+      ic = next;
+    }
   } else {
-    const int ic = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ic < d.nc) update_item<MODE, false>(d, sp, ic, na);
+    if (ic < d.nc) update_item<MODE, false>(d, sp, ic, c, na);
   }
   if (!d.trig_first) pdl_trigger();
   __shared__ __align__(16) unsigned char sh[FVS_NORM_SH_BYTES];
@@ -2796,8 +2837,10 @@ __global__ void __launch_bounds__(256, 2) k_persistent_cell(const DevView d, con
 
 template <int MODE>
 __global__ void __launch_bounds__(256, 2) k_tiles_cell(const DevView d, const PersistPlan p, int k) {
+  pdl_wait();
   const double time = p.t1 + double(*p.step0_dev) * d.dt + p.sp[k].dts;
   cell_stage_tile<MODE>(d, p, p.sp[k], stage_pin(d, k), stage_pout(d, k), blockIdx.x, time);
+  pdl_trigger();
   if (p.sp[k].last) tiled_case_norm(p, blockIdx.x);
 }
 #endif
@@ -2873,21 +2916,34 @@ static cudaError_t launch_persistent(const DevView& d, const PersistPlan& p, int
 template <int LIM>
 __global__ void __launch_bounds__(256) k_tiles_gradient(const DevView d, const PersistPlan p) {
   const int4 tl = p.cell_tiles[blockIdx.x];
+  pdl_wait();
   for (int ic = tl.x + threadIdx.x; ic < tl.y; ic += blockDim.x) gradient_item<FVS_GRAD_LSQ, LIM, false>(d, ic);
+  pdl_trigger();
 }
 
 // ONE: tiles as long as the block, one edge slot or cell per thread (the
 // single-mesh kernels' shape and register budget: no paired slots, no loop)
 template <int REC, bool ONE>
 __global__ void __launch_bounds__(256) k_tiles_flux(const DevView d, const PersistPlan p, int stage) {
-  const double told = p.t1 + double(*p.step0_dev) * d.dt;
   const int2 tl = p.edge_tiles[blockIdx.x];
+  // the stage's time; *step0_dev is the step counter, advanced by the last update
+  auto time = [&]() { return p.t1 + double(*p.step0_dev) * d.dt + p.sp[stage].dts; };
   if (ONE) {
     const int e = tl.x + threadIdx.x;
-    if (e < tl.y) flux_item<REC, false>(d, e, [&]() { return told + p.sp[stage].dts; });
+    FluxItem<REC, false> f;
+    if (e < tl.y) f.load_static(d, e);
+    pdl_wait();
+    if (e < tl.y) {
+      T flux[4], wsa;
+      f.run(d, e, time, flux, wsa);
+      st4(static_cast<T*>(d.eflux), e, flux);
+      static_cast<T*>(d.ews)[e] = wsa;
+    }
   } else {
-    flux_range<REC, false>(d, tl.x + threadIdx.x, tl.y, blockDim.x, told + p.sp[stage].dts);
+    pdl_wait();
+    flux_range<REC, false>(d, tl.x + threadIdx.x, tl.y, blockDim.x, time());
   }
+  pdl_trigger();
 }
 
 template <int MODE, bool ONE>
@@ -2896,11 +2952,17 @@ __global__ void __launch_bounds__(256) k_tiles_update(const DevView d, const Per
   if (ONE) {
     const int4 tl = p.cell_tiles[blockIdx.x];
     const int ic = tl.x + threadIdx.x;
+    CellStatic c;
+    if (ic < tl.y) c.load(d, ic);
+    pdl_wait();
     NormAcc na;
-    if (ic < tl.y) update_item<MODE, false>(d, sp, ic, na);
+    if (ic < tl.y) update_item<MODE, false>(d, sp, ic, c, na);
+    pdl_trigger();
     if (sp.last) tile_norm_partial(p, na, blockIdx.x);
   } else {
+    pdl_wait();
     update_tile<MODE>(d, p, sp, blockIdx.x);
+    pdl_trigger();
   }
   if (sp.last) tiled_case_norm(p, blockIdx.x);
 }
@@ -2911,9 +2973,9 @@ static cudaError_t launch_tiled_step(const DevView& d, const PersistPlan& p, int
   if (cell_fused(d)) {
     for (int k = 0; k < p.nstages; k++) {
       switch (p.sp[k].mode) {
-        case MODE_SSP42: k_tiles_cell<MODE_SSP42><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
-        case MODE_SSP3: k_tiles_cell<MODE_SSP3><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
-        default: k_tiles_cell<MODE_RK><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
+        case MODE_SSP42: launch_k(k_tiles_cell<MODE_SSP42>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
+        case MODE_SSP3: launch_k(k_tiles_cell<MODE_SSP3>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
+        default: launch_k(k_tiles_cell<MODE_RK>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
       }
     }
     return cudaGetLastError();
@@ -2921,27 +2983,27 @@ static cudaError_t launch_tiled_step(const DevView& d, const PersistPlan& p, int
 #endif
   for (int k = 0; k < p.nstages; k++) {
     if (!d.first_order) {
-      if (d.limiter != FVS_LIM_NONE) k_tiles_gradient<1><<<p.ncell_tiles, block, 0, s>>>(d, p);
-      else k_tiles_gradient<0><<<p.ncell_tiles, block, 0, s>>>(d, p);
+      if (d.limiter != FVS_LIM_NONE) launch_k(k_tiles_gradient<1>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p);
+      else launch_k(k_tiles_gradient<0>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p);
     }
     if (one) {
-      if (d.first_order) k_tiles_flux<REC_FIRST, true><<<p.nedge_tiles, block, 0, s>>>(d, p, k);
-      else if (persistent_spec(d)) k_tiles_flux<REC_SPEC, true><<<p.nedge_tiles, block, 0, s>>>(d, p, k);
-      else k_tiles_flux<REC_GENERAL, true><<<p.nedge_tiles, block, 0, s>>>(d, p, k);
+      if (d.first_order) launch_k(k_tiles_flux<REC_FIRST, true>, (unsigned)p.nedge_tiles, (unsigned)block, 0, s, d, p, k);
+      else if (persistent_spec(d)) launch_k(k_tiles_flux<REC_SPEC, true>, (unsigned)p.nedge_tiles, (unsigned)block, 0, s, d, p, k);
+      else launch_k(k_tiles_flux<REC_GENERAL, true>, (unsigned)p.nedge_tiles, (unsigned)block, 0, s, d, p, k);
       switch (p.sp[k].mode) {
-        case MODE_SSP42: k_tiles_update<MODE_SSP42, true><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
-        case MODE_SSP3: k_tiles_update<MODE_SSP3, true><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
-        default: k_tiles_update<MODE_RK, true><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
+        case MODE_SSP42: launch_k(k_tiles_update<MODE_SSP42, true>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
+        case MODE_SSP3: launch_k(k_tiles_update<MODE_SSP3, true>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
+        default: launch_k(k_tiles_update<MODE_RK, true>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
       }
       continue;
     }
-    if (d.first_order) k_tiles_flux<REC_FIRST, false><<<p.nedge_tiles, block, 0, s>>>(d, p, k);
-    else if (persistent_spec(d)) k_tiles_flux<REC_SPEC, false><<<p.nedge_tiles, block, 0, s>>>(d, p, k);
-    else k_tiles_flux<REC_GENERAL, false><<<p.nedge_tiles, block, 0, s>>>(d, p, k);
+    if (d.first_order) launch_k(k_tiles_flux<REC_FIRST, false>, (unsigned)p.nedge_tiles, (unsigned)block, 0, s, d, p, k);
+    else if (persistent_spec(d)) launch_k(k_tiles_flux<REC_SPEC, false>, (unsigned)p.nedge_tiles, (unsigned)block, 0, s, d, p, k);
+    else launch_k(k_tiles_flux<REC_GENERAL, false>, (unsigned)p.nedge_tiles, (unsigned)block, 0, s, d, p, k);
     switch (p.sp[k].mode) {
-      case MODE_SSP42: k_tiles_update<MODE_SSP42, false><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
-      case MODE_SSP3: k_tiles_update<MODE_SSP3, false><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
-      default: k_tiles_update<MODE_RK, false><<<p.ncell_tiles, block, 0, s>>>(d, p, k); break;
+      case MODE_SSP42: launch_k(k_tiles_update<MODE_SSP42, false>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
+      case MODE_SSP3: launch_k(k_tiles_update<MODE_SSP3, false>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
+      default: launch_k(k_tiles_update<MODE_RK, false>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, p, k); break;
     }
   }
   return cudaGetLastError();
@@ -3496,26 +3558,30 @@ static cudaError_t dc_persistent(const DevView& d, const PersistPlan& p, const D
 // spilling
 __global__ void __launch_bounds__(256, 4) k_tiles_dc_flux(const DevView d, const DcView c, const PersistPlan p) {
   const int2 tl = p.edge_tiles[blockIdx.x];
+  pdl_wait();
   dc_flux_range(d, c, tl.x + threadIdx.x, tl.y, blockDim.x);
+  pdl_trigger();
 }
 
 template <int MODE, bool FUSED>
 __global__ void __launch_bounds__(256) k_tiles_dc_update(const DevView d, const DcView c, const PersistPlan p,
                                                          int stage) {
+  pdl_wait();
   dc_stage_tile<MODE, FUSED>(d, c, p, stage, blockIdx.x);
+  pdl_trigger();
   if (p.sp[stage].last) tiled_case_norm(p, blockIdx.x);
 }
 
 static cudaError_t dc_tiled_step(const DevView& d, const PersistPlan& p, const DcView& c, int block, cudaStream_t s) {
   for (int k = 0; k < p.nstages; k++) {
     if (c.dP2) {
-      if (p.sp[k].mode == MODE_SSP42) k_tiles_dc_update<MODE_SSP42, true><<<p.ncell_tiles, block, 0, s>>>(d, c, p, k);
-      else k_tiles_dc_update<MODE_RK, true><<<p.ncell_tiles, block, 0, s>>>(d, c, p, k);
+      if (p.sp[k].mode == MODE_SSP42) launch_k(k_tiles_dc_update<MODE_SSP42, true>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, c, p, k);
+      else launch_k(k_tiles_dc_update<MODE_RK, true>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, c, p, k);
       continue;
     }
-    k_tiles_dc_flux<<<p.nedge_tiles, block, 0, s>>>(d, c, p);
-    if (p.sp[k].mode == MODE_SSP42) k_tiles_dc_update<MODE_SSP42, false><<<p.ncell_tiles, block, 0, s>>>(d, c, p, k);
-    else k_tiles_dc_update<MODE_RK, false><<<p.ncell_tiles, block, 0, s>>>(d, c, p, k);
+    launch_k(k_tiles_dc_flux, (unsigned)p.nedge_tiles, (unsigned)block, 0, s, d, c, p);
+    if (p.sp[k].mode == MODE_SSP42) launch_k(k_tiles_dc_update<MODE_SSP42, false>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, c, p, k);
+    else launch_k(k_tiles_dc_update<MODE_RK, false>, (unsigned)p.ncell_tiles, (unsigned)block, 0, s, d, c, p, k);
   }
   return cudaGetLastError();
 }
