@@ -38,15 +38,6 @@ namespace {
 
 thread_local std::string g_batch_create_error;
 
-__global__ void kb_scatter_in(const double* __restrict__ ref, const int* __restrict__ perm, double* __restrict__ dev, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double2* s = reinterpret_cast<const double2*>(ref) + 2 * (size_t)i;
-  double2* t = reinterpret_cast<double2*>(dev) + 2 * (size_t)perm[i];
-  t[0] = s[0];
-  t[1] = s[1];
-}
-
 __global__ void kb_gather_out(const double* __restrict__ dev, const int* __restrict__ perm, double* __restrict__ ref, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -112,6 +103,7 @@ struct fvs_batch {
   int graph_steps = -1;
   bool plan_dirty = true, use_graph = true;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t evc = nullptr;                  // an upload's copy has left the caller's buffer
   cudaEvent_t eva = nullptr, evb = nullptr;  // around one chunk's launches (shape trials)
   bool retune = true;                         // shape trials as the active set shrinks
   int* h_step0 = nullptr;
@@ -136,6 +128,7 @@ struct fvs_batch {
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (eva) cudaEventDestroy(eva);
+    if (evc) cudaEventDestroy(evc);
     if (evb) cudaEventDestroy(evb);
     if (h_step0) cudaFreeHost(h_step0);
     arena.release();
@@ -623,6 +616,7 @@ int fvs_batch_create(const fvs_mesh* meshes, const fvs_options* opts, int32_t nc
   cudaEventCreate(&B->ev0);
   cudaEventCreate(&B->ev1);
   cudaEventCreate(&B->eva);
+  cudaEventCreateWithFlags(&B->evc, cudaEventDisableTiming);
   cudaEventCreate(&B->evb);
   cudaDeviceGetAttribute(&B->nsm, cudaDevAttrMultiProcessorCount, 0);
   init_view_constants(B.get(), B->d);
@@ -663,12 +657,13 @@ int fvs_batch_set_state(fvs_batch* b, int32_t icase, const double* cvar) {
   const int n = b->cnum[icase];
   cudaError_t e = cudaMemcpyAsync(b->d_stage, cvar, 32 * (size_t)n, cudaMemcpyHostToDevice, b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "state upload");
-  kb_scatter_in<<<(n + 255) / 256, 256, 0, b->stream>>>(b->d_stage, b->d_perm + b->ref_off[icase], b->d.U, n);
-  // primitives with the kernel set's own conversion (the same rounding as
-  // the update kernel produces them)
-  b->ks->cvar2pvar(b->d, b->stream);
-  e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  e = cudaEventRecord(b->evc, b->stream);
+  // with the case's primitives, by the kernel set's own conversion (the same
+  // rounding as the update kernel produces them)
+  b->ks->state_in(b->d, b->d_stage, b->d_perm + b->ref_off[icase], n, b->stream);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  // the caller's buffer is free once the copy has left it
+  if (e == cudaSuccess) e = cudaEventSynchronize(b->evc);
   return e == cudaSuccess ? FVS_OK : b->cuda_fail(e, "set_state");
 }
 
@@ -783,11 +778,10 @@ int fvs_batch_steps(fvs_batch* b, int32_t nsteps, double* norms, float* ms) {
   if ((rc = check_barrier(b))) return rc;
   if (ms) cudaEventElapsedTime(ms, b->ev0, b->ev1);
   if (norms) {
-    std::vector<double> all(4 * (size_t)b->ncases * b->norm_cap);
-    cudaError_t e = cudaMemcpy(all.data(), b->d_case_norms, 8 * all.size(), cudaMemcpyDeviceToHost);
+    // (the stream was synchronised by check_barrier)
+    const cudaError_t e = cudaMemcpy2D(norms, 32 * (size_t)nsteps, b->d_case_norms, 32 * (size_t)b->norm_cap,
+                                       32 * (size_t)nsteps, b->ncases, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return b->cuda_fail(e, "norm download");
-    for (int c = 0; c < b->ncases; c++)
-      std::memcpy(norms + 4 * (size_t)c * nsteps, &all[4 * (size_t)c * b->norm_cap], 32 * (size_t)nsteps);
   }
   return FVS_OK;
 }

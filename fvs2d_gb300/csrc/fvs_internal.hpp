@@ -137,7 +137,7 @@ struct DevView {
   double* norms = nullptr;        // [norm_cap] x 4
   int norm_cap = 0;
   int* bounds_err = nullptr;      // [4] index-checking kernels: flag, site, index, extent
-  int* stepctl = nullptr;         // [0] = steps done in this call
+  int* stepctl = nullptr;         // [0] = steps done in this call; right behind tctl (one upload sets both)
   int trig_first = 0;             // the launch's pdl_trigger before its work (else after it)
   int upd_grid = 0;               // blocks of the last stage's update launch, which strides over the cells
                                   // (one wave of resident blocks; 0: one block per 256 cells)
@@ -290,6 +290,8 @@ struct PersistPlan {
 struct KernelSet {
   const char* name;
   void (*begin_step)(const DevView&, cudaStream_t);  // tile stages: tctl[1]
+  // n cells of a host state (reference order, on the device) to perm[i], with their primitives
+  void (*state_in)(const DevView&, const double* ref, const int* perm, int n, cudaStream_t);
   void (*cvar2pvar)(const DevView&, cudaStream_t);
   void (*gradient)(const DevView&, cudaStream_t);
   // ws_out: also store the wave-speed records (a steady scheme's first stage

@@ -7,7 +7,7 @@
 
 namespace fvs {
 const KernelSet& kernels_fp64_fast() {
-  static const KernelSet k = {"fast", k_fast::launch_begin_step, k_fast::launch_cvar2pvar, k_fast::launch_gradient,
+  static const KernelSet k = {"fast", k_fast::launch_begin_step, k_fast::launch_state_in, k_fast::launch_cvar2pvar, k_fast::launch_gradient,
                               k_fast::launch_flux, k_fast::launch_update, k_fast::launch_residual_out, k_fast::persistent_occupancy,
                               k_fast::launch_persistent, k_fast::launch_tiled_step,
                               nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,

@@ -858,12 +858,23 @@ __device__ __forceinline__ void ghost_state(const DevView& d, int rec, double ti
     const T T_inf = T(d.vinf[3]) / T(d.vinf[0]);
     const T dx = x - (T(d.vx) + T(d.vinf[1]) * T(time));
     const T dy = y - (T(d.vy) + T(d.vinf[2]) * T(time));
+#if FVS_FP64_FAST || FVS_DF
+    // one exponential and one power: exp(1 - r^2) is the square of the first,
+    // and p = rho^gamma = rho T with rho = T^(1/(gamma-1))
+    const T ex = texp_(half(T(1) - (dx * dx + dy * dy)));
+    pfR[1] = T(d.vinf[1]) - q * dy * ex;
+    pfR[2] = T(d.vinf[2]) + q * dx * ex;
+    const T temp = T_inf - (q * q) * (g - T(1)) / (T(2) * g) * (ex * ex);
+    pfR[0] = tpow_(temp, T(1) / (g - T(1)));
+    pfR[3] = pfR[0] * temp;
+#else
     const T r = dsqrt_(dx * dx + dy * dy);
     pfR[1] = T(d.vinf[1]) - q * dy * texp_(T(0.5) * (T(1) - r * r));
     pfR[2] = T(d.vinf[2]) + q * dx * texp_(T(0.5) * (T(1) - r * r));
     const T temp = T_inf - (q * q) * (g - T(1)) / (T(2) * g) * texp_(T(1) - r * r);
     pfR[0] = tpow_(temp, T(1) / (g - T(1)));
     pfR[3] = tpow_(pfR[0], g);
+#endif
   } else {
     // manufactured solution, src/mms.f90:187-213 (values only)
 #pragma unroll
@@ -2531,6 +2542,21 @@ __global__ void __launch_bounds__(256) k_residual_out(const DevView d) {
   d.ws[ic] = ws;
 }
 
+// a host state in reference order (n cells from ref, perm: device cell of each)
+// into the device order, with its primitives
+__global__ void __launch_bounds__(256) k_state_in(const DevView d, const double* __restrict__ ref,
+                                                  const int* __restrict__ perm, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int ic = perm[i];
+  double u[4];
+  T p[4];
+  ld4(ref, i, u);
+  st4(d.U, ic, u);
+  cons2prim(TP(gm1), u, p);
+  st4(static_cast<T*>(d.Pv), ic, p);
+}
+
 __global__ void __launch_bounds__(256) k_cvar2pvar(const DevView d) {
   pdl_wait();
   pdl_trigger();
@@ -3026,6 +3052,9 @@ static inline unsigned grid_for(int n, unsigned block) { return ((unsigned)n + b
 
 
 static void launch_begin_step(const DevView& d, cudaStream_t s) { launch_k(k_begin_step, 1, 1, 0, s, d); }
+static void launch_state_in(const DevView& d, const double* ref, const int* perm, int n, cudaStream_t s) {
+  k_state_in<<<grid_of(n), 256, 0, s>>>(d, ref, perm, n);
+}
 static void launch_cvar2pvar(const DevView& d, cudaStream_t s) { launch_k(k_cvar2pvar, grid_of(d.nc), 256, 0, s, d); }
 
 static void launch_gradient(const DevView& d, cudaStream_t s) {

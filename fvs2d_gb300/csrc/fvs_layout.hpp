@@ -397,8 +397,8 @@ bool alloc_work(DeviceArena& A, DevView& d, int nc, int ne, int nblk, int norm_c
   FVS_ALLOC(ews, void*, sizeof(T) * (size_t)ne);
   FVS_ALLOC(partials, double*, 32 * (size_t)nblk);
   FVS_ALLOC(norms, double*, 32 * (size_t)norm_cap);
-  FVS_ALLOC(stepctl, int*, 16);
-  FVS_ALLOC(tctl, double*, 16);
+  FVS_ALLOC(tctl, double*, 32);
+  d.stepctl = reinterpret_cast<int*>(d.tctl + 2);
 #undef FVS_ALLOC
   return ok;
 }
