@@ -1043,6 +1043,16 @@ __device__ __forceinline__ void face_states(const DevView& d, int e, bool interi
         const T gradR = fma(dr.x, gxr[v], dr.y * gyr[v]);
         pfL[v] = fma(phiL, fma(kh, gradC, omk * gradL), pl[v]);
         pfR[v] = fma(phiR, fma(nkh, gradC, omk * gradR), pr[v]);
+#elif FVS_DF
+        const T gradL = dfma(dl.x, gxl[v], dl.y * gyl[v]);
+        const T gradR = dfma(dr.x, gxr[v], dr.y * gyr[v]);
+        if (d.limiter == FVS_LIM_NONE) {  // phi = 1
+          pfL[v] = dfma(kh, gradC, dfma(omk, gradL, pl[v]));
+          pfR[v] = dfma(nkh, gradC, dfma(omk, gradR, pr[v]));
+        } else {
+          pfL[v] = dfma(phiL, dfma(kh, gradC, omk * gradL), pl[v]);
+          pfR[v] = dfma(phiR, dfma(nkh, gradC, omk * gradR), pr[v]);
+        }
 #else
         const T gradL = dl.x * gxl[v] + dl.y * gyl[v];
         const T gradR = dr.x * gxr[v] + dr.y * gyr[v];
@@ -2963,7 +2973,8 @@ __global__ void __launch_bounds__(256) k_tiles_flux(const DevView d, const Persi
       T flux[4], wsa;
       f.run(d, e, time, flux, wsa);
       st4(static_cast<T*>(d.eflux), e, flux);
-      static_cast<T*>(d.ews)[e] = wsa;
+      // read for the local time step only
+      if (p.sp[stage].steady && p.sp[stage].stage == 1) static_cast<T*>(d.ews)[e] = wsa;
     }
   } else {
     pdl_wait();
