@@ -366,6 +366,7 @@ bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weig
   d.nint = L.nint;
   d.nedge = L.ne;
   d.vol = dvol; d.rvol = drvol; d.cflist = dcf; d.nvrt = dnv;
+  d.st_max = L.ell_n.empty() ? 0 : *std::max_element(L.ell_n.begin(), L.ell_n.end());
   d.ell_base = d_eb; d.ell_n = d_en; d.ell_cell = d_ec; d.ell_coef = t_ell; d.ell_w = t_w;
   d.ecell = dec; d.ebtype = deb; d.volT = t_rvol; d.eps2 = t_eps2; d.cpos = t_cpos;
   d.coef0 = t_c0; d.enrm = t_nrm; d.earea = t_area; d.edL = t_edL; d.edR = t_edR; d.exy = t_exy;
