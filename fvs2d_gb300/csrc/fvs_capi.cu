@@ -30,9 +30,11 @@ thread_local std::string g_create_error;
 
 // Downloads up to this many bytes go through the handle's pinned buffer and a
 // host copy: one transfer for all of a call's arrays, where every copy into
-// pageable memory waits for the device by itself (2,160-cell residual with
-// gradient: 155 -> 120 us a call, with fewer launches).
-constexpr size_t kPinned = 512 << 10;
+// pageable memory waits for the device by itself (residual with gradient of
+// 1,152 cells, FP64: 105 us a call against 120 without).  Above, the host copy into
+// fresh pages costs more than the second transfer (8,192 cells, limits of 128 /
+// 512 KB: 133 / 165 us).
+constexpr size_t kPinned = 128 << 10;
 
 // W values of cell ic as FP64 to out; the device arrays are 16-byte aligned per 4 values
 template <int W, typename V>
