@@ -334,17 +334,28 @@ void launch_tc(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cuda
   cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+template <bool A_KM, bool B_KM, int OUT, int STAGES, int BN>
+void gemm_tc_launch(fvs_mlp* m, const tc::GemmArgs& a) {
+  const dim3 grid((unsigned)((a.N + BN - 1) / BN), (unsigned)((a.M + tc::BM - 1) / tc::BM));
+  launch_tc(tc::k_gemm_tc<A_KM, B_KM, OUT, STAGES, BN>, grid, tc::THREADS, tc::smem_bytes(STAGES, BN), m->stream, a, m->gemm_err);
+}
+
+// With more tiles than two per SM the epilogues of some CTAs run beside the
+// loads of others, and CTAs with two stages, four to an SM, beat two with four
+// (65,536 x 256 x 256 with GELU: 68 / 79 us before the swizzle); below that a
+// CTA has only its own blocks in flight.  A hidden layer whose tiles of 128
+// columns are still that many reads A half as often with them (prediction of
+// 240,000 rows, 256 wide: 686 us, 718 with 64 columns; 112 wide: 365 / 361, so
+// not below a whole tile).
+constexpr bool wide_tiles(int out) { return out == tc::OUT_GELU; }
 template <bool A_KM, bool B_KM, int OUT>
 void gemm_tc(fvs_mlp* m, const tc::GemmArgs& a) {
-  const dim3 grid((unsigned)((a.N + tc::BN - 1) / tc::BN), (unsigned)((a.M + tc::BM - 1) / tc::BM));
-  // With more tiles than two per SM the epilogues of some CTAs run beside the
-  // loads of others, and four CTAs with two stages each beat two with four
-  // (65,536 x 256 x 256 with GELU: 68 / 79 us); below that a CTA has only its
-  // own blocks in flight.
-  if (grid.x * grid.y > 304)
-    launch_tc(tc::k_gemm_tc<A_KM, B_KM, OUT, 2>, grid, tc::THREADS, tc::smem_bytes(2), m->stream, a, m->gemm_err);
-  else
-    launch_tc(tc::k_gemm_tc<A_KM, B_KM, OUT, 4>, grid, tc::THREADS, tc::smem_bytes(4), m->stream, a, m->gemm_err);
+  const long long rows = (a.M + tc::BM - 1) / tc::BM;
+  if constexpr (wide_tiles(OUT)) {
+    if (a.N >= 128 && rows * ((a.N + 127) / 128) > 304) return gemm_tc_launch<A_KM, B_KM, OUT, 2, 128>(m, a);
+  }
+  if (rows * ((a.N + 63) / 64) > 304) gemm_tc_launch<A_KM, B_KM, OUT, 2, 64>(m, a);
+  else gemm_tc_launch<A_KM, B_KM, OUT, 4, 64>(m, a);
 }
 
 template <bool A_KM, bool B_KM>
@@ -356,16 +367,20 @@ void gemm_mma(fvs_mlp* m, const bf16* A, int lda, const bf16* B, int ldb, int M,
 
 // dynamic shared memory of the tcgen05 GEMMs
 template <class Kernel>
-bool tc_smem(Kernel k, int stages) {
-  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::smem_bytes(stages)) == cudaSuccess;
+bool tc_smem(Kernel k, int stages, int bn) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::smem_bytes(stages, bn)) == cudaSuccess;
 }
 template <bool A_KM, bool B_KM, int OUT>
-bool tc_smem_both() {
-  return tc_smem(tc::k_gemm_tc<A_KM, B_KM, OUT, 2>, 2) && tc_smem(tc::k_gemm_tc<A_KM, B_KM, OUT, 4>, 4);
+bool tc_smem_all() {
+  if constexpr (wide_tiles(OUT)) {
+    if (!tc_smem(tc::k_gemm_tc<A_KM, B_KM, OUT, 2, 128>, 2, 128)) return false;
+  }
+  return tc_smem(tc::k_gemm_tc<A_KM, B_KM, OUT, 2, 64>, 2, 64) && tc_smem(tc::k_gemm_tc<A_KM, B_KM, OUT, 4, 64>, 4, 64);
 }
 bool tc_gemm_setup() {
-  return tc_smem_both<true, true, tc::OUT_GELU>() && tc_smem_both<true, true, tc::OUT_PRED>() &&
-         tc_smem_both<true, true, tc::OUT_MSE>() && tc_smem_both<true, false, tc::OUT_DGELU>() && tc_smem(tc::k_grads, 2);
+  return tc_smem_all<true, true, tc::OUT_GELU>() && tc_smem_all<true, true, tc::OUT_PRED>() &&
+         tc_smem_all<true, true, tc::OUT_MSE>() && tc_smem_all<true, false, tc::OUT_DGELU>() &&
+         tc_smem(tc::k_grads, 2, tc::GRAD_BN);
 }
 
 void refresh_bf16(fvs_mlp* m) { k_f32_to_bf16<<<nblk(m->nparam), 256, 0, m->stream>>>(m->w, m->wb, m->nparam); }
@@ -429,7 +444,7 @@ bool grad_plan(fvs_mlp* m, int rows, tc::GradPlan& p) {
     tc::GradLayer& g = p.l[l];
     g.dZ = m->dz[l].p; g.X = m->act[l].p;
     g.din = m->din[l]; g.dout = m->dout[l];
-    g.tiles_n = (g.din + tc::BN - 1) / tc::BN;
+    g.tiles_n = (g.din + tc::GRAD_BN - 1) / tc::GRAD_BN;
     g.tiles = g.tiles_n * ((g.dout + tc::BM - 1) / tc::BM);
     const int square = ((g.din + 127) / 128) * ((g.dout + 127) / 128);
     g.per = nk;
@@ -495,7 +510,7 @@ bool backward(fvs_mlp* m, int n, const tc::AdamArgs* adam) {
   }
   tc::GradPlan p;
   if (!grad_plan(m, n, p)) return false;
-  launch_tc(tc::k_grads, dim3((unsigned)p.ctas), tc::THREADS, tc::smem_bytes(2), m->stream, p,
+  launch_tc(tc::k_grads, dim3((unsigned)p.ctas), tc::THREADS, tc::smem_bytes(2, tc::GRAD_BN), m->stream, p,
             m->part.p, m->gemm_err);
   if (adam)
     launch_tc(tc::k_finish_grads<true>, dim3(nblk(m->nparam)), 256, 0, m->stream, p, (const float*)m->part.p, m->nparam,

@@ -7,22 +7,21 @@
 // aligned (the padded layers of fvs_mlp.cu), so every 16-byte chunk lies
 // wholly inside or outside its matrix.
 //
-// CTA tile 128 x 64, K in blocks of 64 over two or four shared-memory stages
-// (48 or 96 KB).  256 threads (8 warps):
+// CTA tile 128 x 64 or 128 x 128, K in blocks of 64 over two or four shared-
+// memory stages (49, 65 or 97 KB).  256 threads (8 warps):
 //   - all threads bring the next blocks in with 16-byte cp.async, one or three
-//     blocks ahead, straight into the tensor core's canonical layouts without swizzle
-//     (core matrices of 8 rows x 16 bytes); chunks outside the matrix are
-//     zero-filled.  A warp's lanes run over the 8 rows of a core matrix first
-//     (no bank conflicts), then over 64 contiguous bytes of each row;
+//     blocks ahead, straight into the tensor core's canonical layouts with the
+//     128-byte swizzle (stage_block); chunks outside the matrix are zero-filled;
 //   - thread 0 issues the MMAs (tcgen05.mma.cta_group::1.kind::f16, M 128,
-//     N 64, K 16) and commits them to the stage's mbarrier, which frees it;
+//     N 64 or 128, K 16) and commits them to the stage's mbarrier, which frees it;
 //   - warp w reads the accumulator rows of tensor-memory lanes 32 (w % 4)..,
-//     32 columns from 32 (w / 4) (tcgen05.ld): a thread holds 32 consecutive
-//     columns of one row, applies the epilogue and stores 32-byte vectors.
+//     32 columns from 32 (w / 4), of the wider tile also 64 further on
+//     (tcgen05.ld): a thread holds 32 consecutive columns of one row, applies
+//     the epilogue and stores 32-byte vectors.
 // The MLP's layers are 256 wide: with tiles of 128 x 128, two K stages filled
 // between barriers and one warpgroup, a 4096 x 256 x 256 layer ran on 64 CTAs
 // in 48 us, most of it waiting on loads and in the epilogue of 128 outputs a
-// thread; here it runs on 128 CTAs and 32 outputs a thread, in 10 us.
+// thread; 128 CTAs of 32 outputs a thread take 7.7 us (10.3 before the swizzle).
 // Every mbarrier wait is bounded (clock64 budget).  On expiry the kernel sets
 // *err, skips the remaining K blocks and the epilogue, waits for the MMAs it
 // already issued (bounded, up to 9 budgets in all), frees its tensor memory
@@ -38,27 +37,31 @@ namespace tc {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int BM = 128, BN = 64, BK = 64, THREADS = 256;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;  // one stage: 16 + 8 KB
-constexpr int smem_bytes(int stages) { return stages * (A_BYTES + B_BYTES); }
-constexpr uint32_t ACC_COLS = 64;                            // FP32 accumulator 128 x 64
+constexpr int BM = 128, BK = 64, THREADS = 256;
+constexpr int A_BYTES = BM * BK * 2;  // one stage of A: 16 KB; of B: 8 KB per 64 columns
+constexpr int smem_bytes(int stages, int bn) { return stages * (A_BYTES + bn * BK * 2) + 1024; }
 constexpr long long WAIT_BUDGET = 4000000000ll;              // clock cycles (~2 s at 2 GHz)
 
-// Shared-memory matrix descriptor: start address >> 4 (bits 0-13), leading
-// byte offset 128 >> 4 (bits 16-29), stride byte offset 256 >> 4 (bits 32-45),
-// descriptor version 1 (bits 46-47), base offset 0, no swizzle (bits 61-63 = 0).
-// In both canonical layouts used here (put_offset) the two core matrices of a
-// 16-wide K step are 128 bytes apart (leading offset) and the 8-element groups
-// along M or N 256 bytes apart (stride offset).
+// Shared-memory matrix descriptors: start address >> 4 (bits 0-13), leading
+// byte offset >> 4 (bits 16-29), stride byte offset >> 4 (bits 32-45),
+// descriptor version 1 (bits 46-47), 128-byte swizzle (mode 2 in bits 61-63).
+// Both majors keep atoms of 8 lines of 128 bytes, the 16-byte chunk c of line l
+// at c ^ l:
+//  K-major: a line is 64 K of a row; groups of 8 rows 1024 bytes apart (stride
+//  offset), a 16-wide K step 32 bytes on.
+//  MN-major: a line is 64 rows of one k; groups of 8 k 1024 bytes apart (stride
+//  offset), blocks of 64 rows 8192 bytes apart (leading offset), a 16-wide K
+//  step 2048 bytes on.
+template <bool KMAJOR>
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
-         ((uint64_t)1 << 46);
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(KMAJOR ? 1 : 8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A BF16 (bits 7-9
 // = 1), B BF16 (bits 10-12 = 1), no negation, bit 15 / 16: A / B MN-major,
 // N >> 3 (bits 17-22), M >> 4 (bits 24-28).
-template <bool A_KM, bool B_KM>
+template <bool A_KM, bool B_KM, int BN>
 __host__ __device__ constexpr uint32_t idesc() {
   return (1u << 4) | (1u << 7) | (1u << 10) | (A_KM ? 0u : 1u << 15) | (B_KM ? 0u : 1u << 16) |
          ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -87,34 +90,23 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// One operand's block of R rows (M or N) x 64 K into shared memory.  Chunk i
-// of 16 bytes: K-major, 8 consecutive k of row r; MN-major, 8 consecutive rows
-// of one k.  The place of a chunk: K steps of 16 R * 32 bytes apart, in a
-// step the groups of 8 rows 256 apart, the two groups of 8 k 128 apart, and
-// within a core matrix 16 bytes per row (K-major) or per k (MN-major).
+// One operand's block of R rows (M or N) x 64 K into shared memory, laid out as
+// its descriptor says, in copies of 16 bytes: K-major, 8 consecutive k of a row;
+// MN-major, 8 consecutive rows of one k.  A warp's copies are four lines of 128
+// contiguous bytes, and the swizzle spreads them over all banks.  (Without the
+// swizzle a line was 64 bytes: a layer of 65,536 rows and 256 outputs took
+// 60.5 us against 36.2, all weight gradients of a batch of 4,096 23.3 against
+// 17.3.)
 template <bool KMAJOR, int R>
 __device__ __forceinline__ void stage_block(uint32_t s, const bf16* g, int ld, int row0, int rows, int k0, int K) {
 #pragma unroll
   for (int q = 0; q < R * 8 / THREADS; q++) {
-    const int i = q * THREADS + (int)threadIdx.x;
-    const int lo = i & 7;
-    int r, k, off;
-    if (KMAJOR) {
-      // lanes: 8 rows, then 4 chunks along k; then the other 4 chunks, then the next 8 rows
-      const int c = (i >> 3) & 7;
-      r = ((i >> 6) << 3) + lo;
-      k = c << 3;
-      off = (c >> 1) * (R * 32) + (r >> 3) * 256 + (c & 1) * 128 + lo * 16;
-    } else {
-      // lanes: 8 k, then 4 chunks along the rows
-      const int c = (i >> 3) & (R / 8 - 1), kg = (i >> 3) / (R / 8);
-      r = c << 3;
-      k = (kg << 3) + lo;
-      off = (kg >> 1) * (R * 32) + c * 256 + (kg & 1) * 128 + lo * 16;
-    }
+    const int i = q * THREADS + (int)threadIdx.x, c = i & 7, l = i >> 3;
+    // line l: row l (K-major), or k l % 64 of the block l / 64 of 64 rows
+    const int r = KMAJOR ? l : ((l >> 6) << 6) + (c << 3), k = KMAJOR ? c << 3 : l & 63;
     const bool in = row0 + r < rows && k0 + k < K;
     const bf16* src = KMAJOR ? g + (size_t)(row0 + r) * ld + (k0 + k) : g + (size_t)(k0 + k) * ld + (row0 + r);
-    cp_async16(s + off, in ? src : g, in ? 16u : 0u);
+    cp_async16(s + l * 128 + ((c ^ (l & 7)) << 4), in ? src : g, in ? 16u : 0u);
   }
 }
 
@@ -182,20 +174,21 @@ __device__ __forceinline__ void store_bf16(bf16* p, const float* v, int ncol) {
     }
 }
 
-// One 128 x 64 output tile at (m0, n0) over the K blocks [kb0, kb0 + nk).
+// One 128 x BN output tile at (m0, n0) over the K blocks [kb0, kb0 + nk).
 // OUT_RAW sums each run of `per` blocks by itself: the accumulators of the
 // runs lie in two halves of the CTA's tensor memory in turn, so a run's partial
 // goes out (to C, C + run, ...) beside the next one's MMAs.
-template <bool A_KM, bool B_KM, int OUT, int STAGES>
+template <bool A_KM, bool B_KM, int OUT, int STAGES, int BN>
 __device__ __forceinline__ void gemm_tile(const GemmArgs& a, int m0, int n0, int kb0, int nk, int per, size_t run,
                                           int* err) {
-  constexpr uint32_t TMEM_COLS = OUT == OUT_RAW ? 2 * ACC_COLS : ACC_COLS;
+  constexpr int B_BYTES = BN * BK * 2;
+  constexpr uint32_t TMEM_COLS = OUT == OUT_RAW ? 2 * BN : BN;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t mbar[STAGES];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_ok;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = (smem_u32(smem) + 1023u) & ~1023u;  // the swizzle works on address bits
 
   if (tid == 0) {
 #pragma unroll
@@ -228,8 +221,8 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& a, int m0, int n0, int
 #pragma unroll
   for (int kb = 0; kb < STAGES - 1; kb++) load(kb);
   // the accumulator of this warp's 32 rows and 32 columns
-  const int c0 = (warp >> 2) * 32;
-  auto read_acc = [&](uint32_t acc, uint32_t* u) {
+  const int c0 = (warp >> 2) * 32;  // and 64 columns further on for wider tiles
+  auto read_acc = [&](uint32_t acc, int c0, uint32_t* u) {
     const uint32_t taddr = acc + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -242,12 +235,12 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& a, int m0, int n0, int
         : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
   };
-  const int m = m0 + (warp & 3) * 32 + lane, n = n0 + c0;
-  const int ncol = min(32, a.N - n);  // a multiple of 16; <= 0: columns past the matrix
+  const int m = m0 + (warp & 3) * 32 + lane;
   // the partial of run r, once its MMAs are complete
   auto store_run = [&](int r) {
     uint32_t u[32];
-    read_acc(tmem + (uint32_t)(r & 1) * ACC_COLS, u);
+    read_acc(tmem + (uint32_t)(r & 1) * BN, c0, u);
+    const int n = n0 + c0, ncol = min(32, a.N - n);
     if (m < a.M && ncol > 0)
       store_f32(a.C + (size_t)r * run + (size_t)m * a.N + n, reinterpret_cast<const float*>(u), ncol);
   };
@@ -262,13 +255,13 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& a, int m0, int n0, int
       const uint32_t a0 = sbase + (uint32_t)(kb % STAGES) * (A_BYTES + B_BYTES), b0 = a0 + A_BYTES;
       const int steps = min(BK / 16, (a.K - (kb0 + kb) * BK + 15) / 16);
       for (int kk = 0; kk < steps; kk++) {
-        const uint64_t ad = smem_desc(a0 + kk * (BM * 32)), bd = smem_desc(b0 + kk * (BN * 32));
+        const uint64_t ad = smem_desc<A_KM>(a0 + kk * (A_KM ? 32 : 2048)), bd = smem_desc<B_KM>(b0 + kk * (B_KM ? 32 : 2048));
         const uint32_t acc = ((OUT == OUT_RAW ? kb % per > 0 : kb > 0) || kk > 0) ? 1u : 0u;
-        const uint32_t dst = OUT == OUT_RAW ? tmem + (uint32_t)((kb / per) & 1) * ACC_COLS : tmem;
+        const uint32_t dst = OUT == OUT_RAW ? tmem + (uint32_t)((kb / per) & 1) * BN : tmem;
         asm volatile(
             "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
             " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dst),
-            "l"(ad), "l"(bd), "r"(idesc<A_KM, B_KM>()), "r"(acc)
+            "l"(ad), "l"(bd), "r"(idesc<A_KM, B_KM, BN>()), "r"(acc)
             : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
@@ -321,52 +314,58 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& a, int m0, int n0, int
   if (s_ok && OUT == OUT_RAW) {
     if (nk > 0) store_run((nk - 1) / per);
   } else if (s_ok) {
-    uint32_t u[32];
-    read_acc(tmem, u);
-    float v[32], e2 = 0.f;
+    float e2 = 0.f;
+#pragma unroll 1
+    for (int cc = c0; cc < BN; cc += 64) {
+      uint32_t u[32];
+      read_acc(tmem, cc, u);
+      const int n = n0 + cc;
+      const int ncol = min(32, a.N - n);  // a multiple of 16; <= 0: columns past the matrix
+      float v[32];
 #pragma unroll
-    for (int j = 0; j < 32; j++) v[j] = __uint_as_float(u[j]);
-    if (m < a.M && ncol > 0) {
-      const size_t at = (size_t)m * a.N + n;
-      if (OUT == OUT_PRED || OUT == OUT_GELU || OUT == OUT_MSE) {
+      for (int j = 0; j < 32; j++) v[j] = __uint_as_float(u[j]);
+      if (m < a.M && ncol > 0) {
+        const size_t at = (size_t)m * a.N + n;
+        if (OUT == OUT_PRED || OUT == OUT_GELU || OUT == OUT_MSE) {
 #pragma unroll
-        for (int j = 0; j < 32; j++)
-          if (j < ncol) v[j] += a.bias[n + j];
-      }
-      if (OUT == OUT_GELU && a.C) store_f32(a.C + at, v, ncol);
-      if (OUT == OUT_PRED) {
-#pragma unroll
-        for (int j = 0; j < 32; j++)
-          if (n + j < a.nt) a.C[(size_t)m * a.nt + n + j] = v[j];
-      }
-      if (OUT == OUT_GELU) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = gelu_tc(v[j]);
-        store_bf16(a.H + at, v, ncol);
-      }
-      if (OUT == OUT_MSE) {
-        const float* t = a.T + (size_t)(a.idx ? a.idx[m] : m) * a.nt;
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-          float d = 0.f;
-          if (n + j < a.nt) {
-            d = v[j] - t[n + j];
-            e2 += d * d;
-          }
-          v[j] = 2.f * d / float(a.M * a.nt);
+          for (int j = 0; j < 32; j++)
+            if (j < ncol) v[j] += a.bias[n + j];
         }
-        store_bf16(a.H + at, v, ncol);
-      }
-      if (OUT == OUT_DGELU) {
-        float z[32];
+        if (OUT == OUT_GELU && a.C) store_f32(a.C + at, v, ncol);
+        if (OUT == OUT_PRED) {
 #pragma unroll
-        for (int j = 0; j < 32; j++) z[j] = 0.f;
+          for (int j = 0; j < 32; j++)
+            if (n + j < a.nt) a.C[(size_t)m * a.nt + n + j] = v[j];
+        }
+        if (OUT == OUT_GELU) {
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-          if (8 * j < ncol) ld8(a.Z + at + 8 * j, z + 8 * j);
+          for (int j = 0; j < 32; j++) v[j] = gelu_tc(v[j]);
+          store_bf16(a.H + at, v, ncol);
+        }
+        if (OUT == OUT_MSE) {
+          const float* t = a.T + (size_t)(a.idx ? a.idx[m] : m) * a.nt;
 #pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = v[j] * gelu_grad_tc(z[j]);
-        store_bf16(a.H + at, v, ncol);
+          for (int j = 0; j < 32; j++) {
+            float d = 0.f;
+            if (n + j < a.nt) {
+              d = v[j] - t[n + j];
+              e2 += d * d;
+            }
+            v[j] = 2.f * d / float(a.M * a.nt);
+          }
+          store_bf16(a.H + at, v, ncol);
+        }
+        if (OUT == OUT_DGELU) {
+          float z[32];
+#pragma unroll
+          for (int j = 0; j < 32; j++) z[j] = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (8 * j < ncol) ld8(a.Z + at + 8 * j, z + 8 * j);
+#pragma unroll
+          for (int j = 0; j < 32; j++) v[j] = v[j] * gelu_grad_tc(z[j]);
+          store_bf16(a.H + at, v, ncol);
+        }
       }
     }
     if (OUT == OUT_MSE) {
@@ -383,10 +382,11 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& a, int m0, int n0, int
   }
 }
 
-// one GEMM: a CTA per 128 x 64 tile (x along N)
-template <bool A_KM, bool B_KM, int OUT, int STAGES>
-__global__ void __launch_bounds__(THREADS, STAGES == 2 ? (OUT == OUT_DGELU ? 3 : 4) : 2) k_gemm_tc(const GemmArgs a, int* __restrict__ err) {
-  gemm_tile<A_KM, B_KM, OUT, STAGES>(a, (int)blockIdx.y * BM, (int)blockIdx.x * BN, 0, (a.K + BK - 1) / BK, 1, 0, err);
+// one GEMM: a CTA per 128 x BN tile (x along N)
+template <bool A_KM, bool B_KM, int OUT, int STAGES, int BN>
+__global__ void __launch_bounds__(THREADS, BN == 128 ? 3 : STAGES == 2 ? (OUT == OUT_DGELU ? 3 : 4) : 2)
+    k_gemm_tc(const GemmArgs a, int* __restrict__ err) {
+  gemm_tile<A_KM, B_KM, OUT, STAGES, BN>(a, (int)blockIdx.y * BM, (int)blockIdx.x * BN, 0, (a.K + BK - 1) / BK, 1, 0, err);
 }
 
 // All weight gradients of a network, dW_l[n][k] = sum_m dZ_l[m][n] X_l[m][k],
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(THREADS, STAGES == 2 ? (OUT == OUT_DGELU ? 3 :
 // sums added in order by k_finish_grads (deterministic).  A CTA takes `runs`
 // consecutive runs of one 128 x 64 tile; a bias CTA 32 columns of one layer's
 // dZ, each column in 32 interleaved row sums added in order.
-constexpr int MAX_LAYERS = 17, BIAS_COLS = 32;
+constexpr int MAX_LAYERS = 17, BIAS_COLS = 32, GRAD_BN = 64;
 struct GradLayer {
   const bf16* dZ;  // [rows][dout]
   const bf16* X;   // [rows][din]
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(THREADS, 4) k_grads(const GradPlan p, float* _
     const size_t run = (size_t)g.dout * g.din;
     a.C = part + g.part + (size_t)z * run;
     const int nk = (p.rows + BK - 1) / BK, kb0 = z * g.per;
-    gemm_tile<false, false, OUT_RAW, 2>(a, tile / g.tiles_n * BM, tile % g.tiles_n * BN, kb0,
+    gemm_tile<false, false, OUT_RAW, 2, GRAD_BN>(a, tile / g.tiles_n * BM, tile % g.tiles_n * GRAD_BN, kb0,
                                      max(0, min(nk - kb0, p.runs * g.per)), g.per, run, err);
     return;
   }

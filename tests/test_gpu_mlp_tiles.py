@@ -39,3 +39,21 @@ def test_tile_edges(n_in, width, depth, n_out):
         d = np.linalg.norm(got["tcgen05"] - got["mma.sync"])
         assert d <= 5e-4 * np.linalg.norm(got["mma.sync"]), n
     m.close()
+
+
+@pytest.mark.parametrize("n_in,width,depth,n", [(8, 128, 2, 39100), (5, 112, 1, 38913), (17, 144, 2, 30001), (5, 256, 1, 65537)])
+def test_wide_tiles(n_in, width, depth, n):
+    """Predictions of enough rows for the hidden layers' 128-column tiles, whole
+    and ragged in rows and columns: both engines against each other."""
+    rng = np.random.default_rng(width)
+    m = MLP(n_in, width, depth, 3, seed=2)
+    x = rng.standard_normal((n, n_in)).astype(np.float32)
+    got = {}
+    for engine in ("tcgen05", "mma.sync"):
+        m.set_engine(engine)
+        got[engine] = m.predict(x)
+    d = np.linalg.norm(got["tcgen05"] - got["mma.sync"], axis=1)
+    # the bar of the tile test, and row by row with the margin of a BF16 rounding
+    assert np.linalg.norm(d) <= 5e-4 * np.linalg.norm(got["mma.sync"])
+    assert d.max() <= 2.0 ** -7 * np.linalg.norm(got["mma.sync"], axis=1).max()
+    m.close()
