@@ -110,7 +110,7 @@ struct DevView {
   // gradient stencil interleaved over groups of 32 cells: entry j of cell ic
   // at ell_base[ic / 32] + 32 j + ic % 32, j < ell_n[ic]
   const int* ell_base = nullptr;
-  const uint8_t* ell_n = nullptr;
+  const uint16_t* ell_n = nullptr;
   int st_max = 0;                  // longest stencil
   const int* ell_cell = nullptr;
   const void* ell_coef = nullptr;  // x 2 (T); GGNB: edge times node coefficient

@@ -135,7 +135,7 @@ struct Layout {
   // the stencil interleaved over groups of 32 cells (build_ell): per group as
   // many rows of 32 entries as its longest stencil has
   std::vector<int> ell_base, ell_cell;
-  std::vector<uint8_t> ell_n;
+  std::vector<uint16_t> ell_n;  // (a stencil of n cells around one node occurs n times: 65,535 is beyond any 32-bit total)
   std::vector<T> ell_coef, ell_w;
 
   // from the CSR rows, entry order kept; places beyond a cell's own entries
@@ -150,8 +150,8 @@ struct Layout {
       int width = 0;
       for (int ic = 32 * g; ic < std::min(nc, 32 * g + 32); ic++) {
         const int n = st_ptr[ic + 1] - st_ptr[ic];
-        if (n > 255) return false;
-        ell_n[ic] = (uint8_t)n;
+        if (n > 65535) return false;
+        ell_n[ic] = (uint16_t)n;
         width = std::max(width, n);
       }
       total += 32LL * width;
@@ -333,7 +333,7 @@ bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weig
   int4* dcf;
   int8_t *dnv, *dsn;
   int *dsp, *deb, *d_eb, *d_ec;
-  uint8_t* d_en;
+  uint16_t* d_en;
   int2* dec;
   T *t_rvol, *t_eps2, *t_cpos, *t_coef, *t_w = nullptr, *t_c0, *t_ce, *t_ell, *t_nrm, *t_area, *t_edL, *t_edR, *t_exy;
   ok = ok && A.upload(dvol, L.vol) && A.upload(drvol, L.rvol) && A.upload(dcf, L.cf) && A.upload(dnv, L.nvrt);
