@@ -349,13 +349,11 @@ bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weig
   }
   if (ok && std::is_same<T, double>::value && !weights) {
     // FP64 kernels: the flux's factors of a face
-    std::vector<double> fac(4 * (size_t)L.ne);
+    std::vector<double> fac(2 * (size_t)L.ne);
     for (size_t e = 0; e < (size_t)L.ne; e++) {
       const double h = 0.5 * double(L.earea[e]);
-      fac[4 * e] = double(L.enrm[2 * e]) * h;
-      fac[4 * e + 1] = double(L.enrm[2 * e + 1]) * h;
-      fac[4 * e + 2] = h;
-      fac[4 * e + 3] = 0.5 * h;
+      fac[2 * e] = double(L.enrm[2 * e]) * h;
+      fac[2 * e + 1] = h;
     }
     double* p = nullptr;
     ok = A.upload(p, fac);
