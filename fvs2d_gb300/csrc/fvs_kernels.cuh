@@ -462,9 +462,10 @@ __device__ __forceinline__ void roe_flux_fast(T gamma, T gm1, T igm1, const T* p
 //  - acoustic strengths doubled (A - B and A + B with A = dp/a^2, B = rho dun/a),
 //    factors of 1/2 folded into the face length
 //  - Harten's fix behind a branch, its compare on the integer pipe
-// With the face states 112 FP64 operations per edge (116 issued) against 134 when
-// the average was formed in x and y from 1/rhoL, 1/rhoR and 1/(1+RT):
-// 1,048,576 cells 393 -> 334 us a launch, the FP64 pipe 88 % busy in both.
+//  - factors of 2 and 1/2 by the exponent, on the integer pipe
+// With the face states 115 FP64 instructions per edge against 134 when the
+// average was formed in x and y from 1/rhoL, 1/rhoR and 1/(1+RT): 1,048,576
+// cells 393 -> 330 us a launch, the FP64 pipe 88 % busy in both.
 // Rounding-level differences to the source form, checked against the oracle
 // at 1e-12.
 __device__ __forceinline__ double harten(double x) {
