@@ -521,15 +521,23 @@ bool backward(fvs_mlp* m, int n, const tc::AdamArgs* adam) {
   return true;
 }
 
+// the call's launches and copies are complete when it returns, with or without an error
 int check(fvs_mlp* m, const char* where) {
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+  const cudaError_t es = cudaStreamSynchronize(m->stream);
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return m->fail(FVS_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
   int flag = 0;
   e = cudaMemcpy(&flag, m->gemm_err, sizeof flag, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return m->fail(FVS_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
   if (flag) return m->fail(FVS_ERR_TIMEOUT, std::string(where) + ": a tensor-core GEMM wait ran out of its budget");
   return FVS_OK;
+}
+
+// an allocation of a call that has copies from the caller's arrays in flight failed
+int fail_in_flight(fvs_mlp* m, const char* what) {
+  cudaStreamSynchronize(m->stream);
+  return m->fail(FVS_ERR_NOMEM, what);
 }
 
 }  // namespace
@@ -675,7 +683,7 @@ int fvs_mlp_loss_grad(fvs_mlp* m, const float* x, const float* y, int32_t n, flo
   if (m->engine == 1) cudaMemsetAsync(m->g, 0, 4 * m->nparam, m->stream);
   k_gather_rows<<<nblk((size_t)n * m->in_pad), 256, 0, m->stream>>>(m->data_x.p, m->n_in, nullptr, n, m->act[0].p, m->in_pad);
   forward(m, n, m->data_y.p, nullptr, nullptr);
-  if (!backward(m, n, nullptr)) return m->fail(FVS_ERR_NOMEM, "gradient workspace");
+  if (!backward(m, n, nullptr)) return fail_in_flight(m, "gradient workspace");
   int rc = check(m, "loss_grad");
   if (rc) return rc;
   float l = 0.f;
@@ -699,17 +707,19 @@ int fvs_mlp_train(fvs_mlp* m, const float* x, const float* y, int64_t n, int32_t
     return m->fail(FVS_ERR_NOMEM, "dataset allocation");
   cudaMemcpyAsync(m->data_x.p, x, 4 * (size_t)n * m->n_in, cudaMemcpyHostToDevice, m->stream);
   cudaMemcpyAsync(m->data_y.p, y, 4 * (size_t)n * m->n_out, cudaMemcpyHostToDevice, m->stream);
-  std::vector<int> idx(n);
+  // Orders of the even and of the odd epochs: one is written while the copy of
+  // the other may still be in flight (an asynchronous copy from pageable memory
+  // may read it after the call has returned); check() ends every epoch.
+  std::vector<int> order[2] = {std::vector<int>(n), std::vector<int>(epochs > 1 ? n : 0)};
   std::mt19937_64 rng(seed);
-  auto shuffle = [&]() {
+  auto shuffle = [&](std::vector<int>& idx) {
     for (int64_t i = 0; i < n; i++) idx[i] = (int)i;
     std::shuffle(idx.begin(), idx.end(), rng);
   };
-  shuffle();
+  shuffle(order[0]);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   for (int ep = 0; ep < epochs; ep++) {
-    // (pageable: copied out of idx when the call returns)
-    cudaMemcpyAsync(m->data_idx.p, idx.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, m->stream);
+    cudaMemcpyAsync(m->data_idx.p, order[ep & 1].data(), 4 * (size_t)n, cudaMemcpyHostToDevice, m->stream);
     cudaMemsetAsync(m->loss, 0, 4, m->stream);
     for (int64_t s0 = 0; s0 + batch <= n; s0 += batch) {
       const int* bi = m->data_idx.p + s0;
@@ -718,9 +728,9 @@ int fvs_mlp_train(fvs_mlp* m, const float* x, const float* y, int64_t n, int32_t
       forward(m, batch, m->data_y.p, bi, nullptr);
       m->step++;
       const tc::AdamArgs ad = {lr, b1, b2, eps, 1.f - std::pow(b1, (float)m->step), 1.f - std::pow(b2, (float)m->step)};
-      if (!backward(m, batch, &ad)) return m->fail(FVS_ERR_NOMEM, "gradient workspace");
+      if (!backward(m, batch, &ad)) return fail_in_flight(m, "gradient workspace");
     }
-    if (ep + 1 < epochs) shuffle();  // the next epoch's order, beside this epoch's steps
+    if (ep + 1 < epochs) shuffle(order[(ep + 1) & 1]);  // the next epoch's order, beside this epoch's steps
     int rc = check(m, "train");
     if (rc) return rc;
     if (loss_per_epoch) {
