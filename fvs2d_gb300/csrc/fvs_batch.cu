@@ -173,10 +173,10 @@ int build_batch_device(fvs_batch* B, DevView& d) {
   if (!alloc_work<T>(B->arena, d, L.nc, L.ne, (L.nc + 255) / 256, 16))
     return B->fail(FVS_ERR_NOMEM, "device allocation of the batch state failed");
   std::vector<T> phi0(L.nc, T(d.first_order ? 0.0 : 1.0));
-  if (cudaMemcpy(d.phi, phi0.data(), sizeof(T) * L.nc, cudaMemcpyHostToDevice) != cudaSuccess)
+  if (upload_sync(d.phi, phi0.data(), sizeof(T) * L.nc) != cudaSuccess)
     return B->fail(FVS_ERR_CUDA, "phi upload failed");
   std::vector<double> dtl(L.nc, B->base.dt);
-  if (cudaMemcpy(d.dtl, dtl.data(), 8 * dtl.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+  if (upload_sync(d.dtl, dtl.data(), 8 * dtl.size()) != cudaSuccess)
     return B->fail(FVS_ERR_CUDA, "dt upload failed");
   return FVS_OK;
 }
@@ -316,10 +316,16 @@ int build_plan(fvs_batch* B) {
     B->d_edge_tiles = static_cast<int2*>(p);
     B->cap_edge_tiles = cap;
   }
+  // in the order of the batch's stream, whose kernels read them; the lists live
+  // until the copies have left them
   cudaError_t e = cudaSuccess;
-  if (!ct.empty()) e = cudaMemcpy(B->d_cell_tiles, ct.data(), 16 * ct.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !et.empty()) e = cudaMemcpy(B->d_edge_tiles, et.data(), 8 * et.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !cases.empty()) e = cudaMemcpy(B->d_case_tiles, cases.data(), 16 * cases.size(), cudaMemcpyHostToDevice);
+  if (!ct.empty()) e = cudaMemcpyAsync(B->d_cell_tiles, ct.data(), 16 * ct.size(), cudaMemcpyHostToDevice, B->stream);
+  if (e == cudaSuccess && !et.empty())
+    e = cudaMemcpyAsync(B->d_edge_tiles, et.data(), 8 * et.size(), cudaMemcpyHostToDevice, B->stream);
+  if (e == cudaSuccess && !cases.empty())
+    e = cudaMemcpyAsync(B->d_case_tiles, cases.data(), 16 * cases.size(), cudaMemcpyHostToDevice, B->stream);
+  const cudaError_t es = cudaStreamSynchronize(B->stream);
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return B->cuda_fail(e, "plan upload");
   PersistPlan& P = B->plan;
   P.tile = B->tile;

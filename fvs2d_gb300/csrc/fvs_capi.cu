@@ -358,7 +358,7 @@ int build_device(fvs_handle* H) {
   H->d_stage = static_cast<double*>(p);
   // phi: 0 for first order, 1 without a limiter (src/gradient_limiter.f90:30-40)
   std::vector<T> phi0(L.nc, T(H->o.reconst == FVS_RECON_UPWIND1 ? 0.0 : 1.0));
-  if (cudaMemcpy(d.phi, phi0.data(), sizeof(T) * L.nc, cudaMemcpyHostToDevice) != cudaSuccess)
+  if (upload_sync(d.phi, phi0.data(), sizeof(T) * L.nc) != cudaSuccess)
     return H->fail(FVS_ERR_CUDA, "phi upload failed");
   if (fuse && H->ks->tile_stage) {
     TilePlan P;
@@ -468,7 +468,8 @@ int bounds_report(fvs_handle* H) {
   if (e != cudaSuccess) return H->cuda_fail(e, "bounds word download");
   if (!w[0]) return FVS_OK;
   static const char* site[] = {"?", "stencil cell", "edge left cell", "edge right cell", "gather slot"};
-  cudaMemset(H->d.bounds_err, 0, sizeof w);
+  e = zero_sync(H->d.bounds_err, sizeof w);
+  if (e != cudaSuccess) return H->cuda_fail(e, "bounds word reset");
   return H->fail(FVS_ERR_BOUNDS, std::string("index-checking kernels: ") + site[(w[1] >= 1 && w[1] <= 4) ? w[1] : 0] +
                                      " index " + std::to_string(w[2]) + " outside its array of " + std::to_string(w[3]));
 }
@@ -688,7 +689,8 @@ int fvs_create(const fvs_mesh* mesh, const fvs_options* opt, fvs_handle** out) {
   // steady runs start from dt_local = dt (src/runge_kutta.f90:73-76)
   {
     std::vector<double> dtl(H->hm.nc, H->o.dt);
-    cudaMemcpy(d.dtl, dtl.data(), 8 * dtl.size(), cudaMemcpyHostToDevice);
+    e = upload_sync(d.dtl, dtl.data(), 8 * dtl.size());
+    if (e != cudaSuccess) { g_create_error = std::string("dt upload: ") + cudaGetErrorString(e); return FVS_ERR_CUDA; }
   }
   if (!(H->o.dt_from_cfl && !H->o.steady)) {
     set_stages(H.get());
@@ -827,7 +829,8 @@ int dma_report(fvs_handle* h) {
   cudaError_t e = cudaMemcpy(&w, h->dv.err, sizeof w, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return h->cuda_fail(e, "bulk-copy error word download");
   if (!w) return FVS_OK;
-  cudaMemset(h->dv.err, 0, sizeof w);
+  e = zero_sync(h->dv.err, sizeof w);
+  if (e != cudaSuccess) return h->cuda_fail(e, "bulk-copy error word reset");
   h->gb_stale = true;
   return h->fail(FVS_ERR_TIMEOUT, "a tile block's wait for its bulk copies ran out");
 }
@@ -1090,7 +1093,7 @@ int fvs_debug_set_gather(fvs_handle* h, int32_t cell, int32_t entry, int32_t val
   int* p = reinterpret_cast<int*>(const_cast<int4*>(h->d.cflist) + h->perm[cell - 1]) + entry;
   // the kernels read the list from memory at every launch, so a captured
   // step graph sees the new entry
-  cudaError_t e = cudaMemcpy(p, &value, sizeof value, cudaMemcpyHostToDevice);
+  cudaError_t e = upload_sync(p, &value, sizeof value);
   return e == cudaSuccess ? FVS_OK : h->cuda_fail(e, "gather entry upload");
 }
 
@@ -1132,7 +1135,7 @@ int fvs_check_fp64_math(const double* x, int32_t n, double* out) {
   double* d = nullptr;
   const size_t nb = sizeof(double) * (size_t)n;
   if (cudaMalloc(&d, 6 * nb) != cudaSuccess) return FVS_ERR_NOMEM;
-  cudaError_t e = cudaMemcpy(d, x, nb, cudaMemcpyHostToDevice);
+  cudaError_t e = upload_sync(d, x, nb);
   if (e == cudaSuccess) {
     k_check_fp64_math<<<(n + 255) / 256, 256>>>(d, n, d + n);
     e = cudaGetLastError();

@@ -22,6 +22,19 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Host data, and zeros, in device memory when the call returns.  A cudaMemcpy
+// from pageable memory may return once its source is staged, and a cudaMemset
+// returns at once; the handles' streams are non-blocking, so their kernels are
+// not ordered behind what the legacy stream still has to do.
+inline cudaError_t upload_sync(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+inline cudaError_t zero_sync(void* dst, size_t bytes) {
+  const cudaError_t e = cudaMemset(dst, 0, bytes);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+
 // ---------------------------------------------------------------------------
 // Host mesh in the reference's numbering, 0-based, "-1" where the reference
 // stores 0 (no neighbour / boundary).  Built by build_host_mesh() so that

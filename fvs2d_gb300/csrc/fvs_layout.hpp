@@ -36,7 +36,7 @@ struct DeviceArena {
     void* p = nullptr;
     if (cudaMalloc(&p, sizeof(V) * src.size()) != cudaSuccess) return false;
     allocs.push_back(p);
-    if (cudaMemcpy(p, src.data(), sizeof(V) * src.size(), cudaMemcpyHostToDevice) != cudaSuccess) return false;
+    if (upload_sync(p, src.data(), sizeof(V) * src.size()) != cudaSuccess) return false;
     dst = static_cast<V*>(p);
     return true;
   }
@@ -45,7 +45,7 @@ struct DeviceArena {
     if (bytes == 0) bytes = 16;
     if (cudaMalloc(&dst, bytes) != cudaSuccess) return false;
     allocs.push_back(dst);
-    return cudaMemset(dst, 0, bytes) == cudaSuccess;
+    return zero_sync(dst, bytes) == cudaSuccess;
   }
 };
 

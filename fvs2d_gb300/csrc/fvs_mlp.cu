@@ -294,8 +294,8 @@ struct fvs_mlp {
   V* dalloc(size_t n) {
     void* p = nullptr;
     if (cudaMalloc(&p, sizeof(V) * std::max<size_t>(n, 1)) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, sizeof(V) * std::max<size_t>(n, 1));
     owned.push_back(p);
+    if (cudaMemsetAsync(p, 0, sizeof(V) * std::max<size_t>(n, 1), stream) != cudaSuccess) return nullptr;
     return static_cast<V*>(p);
   }
   // layer buffers for `rows` rows; train: those of the backward pass too
@@ -597,7 +597,7 @@ int fvs_mlp_create(int32_t n_in, int32_t width, int32_t depth, int32_t n_out, ui
     for (int r = 0; r < rows; r++)
       for (int k = 0; k < fan_in; k++) h[m->woff[l] + (size_t)r * m->din[l] + k] = nd(rng);
   }
-  cudaMemcpy(m->w, h.data(), 4 * off, cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(m->w, h.data(), 4 * off, cudaMemcpyHostToDevice, m->stream);
   refresh_bf16(m.get());
   if (check(m.get(), "MLP init")) {
     g_mlp_error = m->err;
@@ -650,8 +650,8 @@ static int copy_params(fvs_mlp* m, float* host, const float* in, int64_t n, bool
     }
   }
   if (!get) {
-    if (cudaMemcpy(m->w, pad.data(), 4 * m->nparam, cudaMemcpyHostToDevice) != cudaSuccess)
-      return m->fail(FVS_ERR_CUDA, "parameter upload");
+    // (check() waits for the copy)
+    cudaMemcpyAsync(m->w, pad.data(), 4 * m->nparam, cudaMemcpyHostToDevice, m->stream);
     cudaMemsetAsync(m->am, 0, 4 * m->nparam, m->stream);
     cudaMemsetAsync(m->av, 0, 4 * m->nparam, m->stream);
     m->step = 0;
