@@ -103,7 +103,6 @@ struct fvs_batch {
   int graph_steps = -1;
   bool plan_dirty = true, use_graph = true;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  cudaEvent_t evc = nullptr;                  // an upload's copy has left the caller's buffer
   cudaEvent_t eva = nullptr, evb = nullptr;  // around one chunk's launches (shape trials)
   bool retune = true;                         // shape trials as the active set shrinks
   int* h_step0 = nullptr;
@@ -128,7 +127,6 @@ struct fvs_batch {
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (eva) cudaEventDestroy(eva);
-    if (evc) cudaEventDestroy(evc);
     if (evb) cudaEventDestroy(evb);
     if (h_step0) cudaFreeHost(h_step0);
     arena.release();
@@ -622,7 +620,6 @@ int fvs_batch_create(const fvs_mesh* meshes, const fvs_options* opts, int32_t nc
   cudaEventCreate(&B->ev0);
   cudaEventCreate(&B->ev1);
   cudaEventCreate(&B->eva);
-  cudaEventCreateWithFlags(&B->evc, cudaEventDisableTiming);
   cudaEventCreate(&B->evb);
   cudaDeviceGetAttribute(&B->nsm, cudaDevAttrMultiProcessorCount, 0);
   init_view_constants(B.get(), B->d);
@@ -663,13 +660,12 @@ int fvs_batch_set_state(fvs_batch* b, int32_t icase, const double* cvar) {
   const int n = b->cnum[icase];
   cudaError_t e = cudaMemcpyAsync(b->d_stage, cvar, 32 * (size_t)n, cudaMemcpyHostToDevice, b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "state upload");
-  e = cudaEventRecord(b->evc, b->stream);
   // with the case's primitives, by the kernel set's own conversion (the same
   // rounding as the update kernel produces them)
   b->ks->state_in(b->d, b->d_stage, b->d_perm + b->ref_off[icase], n, b->stream);
-  if (e == cudaSuccess) e = cudaGetLastError();
-  // the caller's buffer is free once the copy has left it
-  if (e == cudaSuccess) e = cudaEventSynchronize(b->evc);
+  e = cudaGetLastError();
+  const cudaError_t es = cudaStreamSynchronize(b->stream);
+  if (e == cudaSuccess) e = es;
   return e == cudaSuccess ? FVS_OK : b->cuda_fail(e, "set_state");
 }
 

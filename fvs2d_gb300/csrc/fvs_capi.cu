@@ -142,7 +142,6 @@ struct fvs_handle {
   int* d_perm = nullptr;   // device copy of perm
   double* d_stage = nullptr;  // [nc][8] reference-order staging
   double* h_small = nullptr;  // pinned: control words, then staging of small downloads
-  cudaEvent_t evc = nullptr;  // an upload's copy has left the caller's buffer
   std::vector<StageParams> stages;
   double dt = 0;
   bool dt_ready = false;
@@ -175,7 +174,6 @@ struct fvs_handle {
     if (graph) cudaGraphExecDestroy(graph);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
-    if (evc) cudaEventDestroy(evc);
     arena.release();
     if (h_small) cudaFreeHost(h_small);
     if (stream) cudaStreamDestroy(stream);
@@ -515,19 +513,18 @@ int ensure_dt(fvs_handle* H, double t1) {
   return FVS_OK;
 }
 
-// the caller's state onto the device; returns once it has left the caller's
-// buffer (the kernels behind the copy run on)
+// the caller's state onto the device; complete at return (fvs_device_state has
+// given callers the array)
 int state_in(fvs_handle* H, const double* cvar) {
   NvtxRange nv("fvs state upload");
   const size_t bytes = 32 * (size_t)H->hm.nc;
   cudaError_t e = cudaMemcpyAsync(H->d_stage, cvar, bytes, cudaMemcpyHostToDevice, H->stream);
-  if (e == cudaSuccess) e = cudaEventRecord(H->evc, H->stream);
   if (e != cudaSuccess) return H->cuda_fail(e, "state upload");
   H->ks->state_in(H->d, H->d_stage, H->d_perm, H->hm.nc, H->stream);
   H->gb_stale = true;
-  int rc = check_launch(H, "state scatter");
-  if (rc) return rc;
-  e = cudaEventSynchronize(H->evc);
+  e = cudaGetLastError();
+  const cudaError_t es = cudaStreamSynchronize(H->stream);
+  if (e == cudaSuccess) e = es;
   return e == cudaSuccess ? FVS_OK : H->cuda_fail(e, "set_state");
 }
 
@@ -653,7 +650,6 @@ int fvs_create(const fvs_mesh* mesh, const fvs_options* opt, fvs_handle** out) {
   if (cudaMallocHost(&H->h_small, 64 + kPinned) != cudaSuccess) { g_create_error = "pinned allocation failed"; return FVS_ERR_NOMEM; }
   cudaEventCreate(&H->ev0);
   cudaEventCreate(&H->ev1);
-  cudaEventCreateWithFlags(&H->evc, cudaEventDisableTiming);
   DevView& d = H->d;
   d.gamma = H->o.gamma;
   d.khalf = H->o.umuscl / 2.0;

@@ -185,6 +185,8 @@ int fvs_export(const fvs_handle* h, const char* name, void* dst, int64_t nbytes)
  * restart from the cont.cd / cont.s8 files, src/initialize.f90:56-77) returns
  * FVS_ERR_INVALID: the host reads the files and calls fvs_set_state. */
 int fvs_init_state(fvs_handle* h);
+/* The state is on the device when the call returns, and an error of its
+ * kernels is this call's. */
 int fvs_set_state(fvs_handle* h, const double* cvar);   /* [ncells][4] */
 int fvs_get_state(fvs_handle* h, double* cvar);         /* [ncells][4] */
 
@@ -232,7 +234,9 @@ int fvs_profile_step(fvs_handle* h, int32_t cap, int32_t* n, char* names /*[cap]
 /* Number of kernel launches one step issues. */
 int fvs_launches_per_step(const fvs_handle* h, int32_t* n);
 /* Device pointer of the conservative state (RCM order) and the permutation
- * old->new (host copy, 0-based) for callers that keep data on the device. */
+ * old->new (host copy, 0-based) for callers that keep data on the device.
+ * Calls on the handle end with their work on the array complete, so between
+ * calls any stream may read it. */
 int fvs_device_state(fvs_handle* h, void** dptr);
 /* Index-checking kernels (no counterpart in the reference, which has no
  * sanitizer either).  With the environment variable FVS2D_BOUNDS=1 at
