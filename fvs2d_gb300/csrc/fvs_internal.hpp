@@ -138,7 +138,6 @@ struct DevView {
   const int2* ecell = nullptr;    // (L,R) device cell ids; R = -1 on boundary edges
   const void* enrm = nullptr;     // [nedge] x 2 unit normal (T)
   const void* earea = nullptr;    // [nedge] (T)
-  const double* efac = nullptr;   // [nedge] x 2: length / 2 times (nx, 1) (FP64 build's flux)
   const void* edL = nullptr;      // [nedge] x 2 xf - xcL (T)
   const void* edR = nullptr;      // [nint] x 2 xf - xcR (T)
   const int* ebtype = nullptr;    // [nedge] boundary record: type | case << 4 (boundary slots only)

@@ -449,12 +449,15 @@ __device__ __forceinline__ void roe_flux_fast(T gamma, T gm1, T igm1, const T* p
 // The Roe flux of roe_flux_fast_t arranged for the FP64 pipe (FVS_PREC_FP64;
 // GB300 issues 2 FP64 operations per clock per SM, and this function is most
 // of the FP64 step):
-//  - everything in the face's frame: normal and tangential velocities of the
-//    two states and of the average, the momentum flux turned back at the end
+//  - average and dissipation in the face's frame (normal and tangential
+//    velocities), the dissipation turned back at the end; the two states' own
+//    momentum and kinetic energy stay in x and y, whose components carry no
+//    rounding of a turn (with the whole momentum turned back its error was
+//    1.1 to 1.3 times the source form's, so it is 0.7 to 0.85 of it)
 //  - the Roe average with density weights: with g = rhoL rhoR and 1/sqrt(g)
 //    the averaged density is sqrt(g), the weights rhoL and sqrt(g), and one
 //    reciprocal of their sum serves all three averages; rho H enters as
-//    2 rho H = rho un^2 + rho ut^2 + 2 gamma/(gamma-1) p, so no state's own
+//    2 rho H = rho (u^2 + v^2) + 2 gamma/(gamma-1) p, so no state's own
 //    density is divided by
 //  - reciprocals and square roots from the hardware approximations refined by
 //    one Newton-Raphson step (fp64_fast.cuh): 1/sqrt(g), 1/(rhoL + sqrt(g)) and
@@ -463,9 +466,8 @@ __device__ __forceinline__ void roe_flux_fast(T gamma, T gm1, T igm1, const T* p
 //    factors of 1/2 folded into the face length
 //  - Harten's fix behind a branch, its compare on the integer pipe
 //  - factors of 2 and 1/2 by the exponent, on the integer pipe
-// With the face states 115 FP64 instructions per edge against 134 when the
-// average was formed in x and y from 1/rhoL, 1/rhoR and 1/(1+RT): 1,048,576
-// cells 393 -> 330 us a launch, the FP64 pipe 88 % busy in both.
+// With the face states 117 FP64 instructions per edge against 134 when the
+// average was formed in x and y from 1/rhoL, 1/rhoR and 1/(1+RT).
 // Rounding-level differences to the source form, checked against the oracle
 // at 1e-12.
 __device__ __forceinline__ double harten(double x) {
@@ -487,23 +489,21 @@ __device__ __forceinline__ double scale2(double x) {
   const bool in = (unsigned)((hi >> 20 & 0x7ff) - 2) < 0x7fcu;
   return __hiloint2double(hi + (in ? K * 0x00100000 : 0), __double2loint(x));
 }
-// hgm1 = (gamma-1)/2, c2 = 2 gamma/(gamma-1); s: the face's factors, l / 2 (nx, 1) with l its length.
-// (Storing l / 2 (nx, ny, 1, 1/2) saves the product ny l / 2, but 16 bytes more per edge are read:
-// 274 MB of DRAM traffic a launch on 1,048,576 cells against 248.)
-struct Area { double hx, h; };
+// hgm1 = (gamma-1)/2, c2 = 2 gamma/(gamma-1); af: the face's length
 __device__ __forceinline__ void roe_flux_area_fp64(double hgm1, double c2, const double* pl, const double* pr,
-                                                   double nx, double ny, Area s, double* flux, double& wsa) {
-  const double rhoL = pl[0], pL = pl[3], rhoR = pr[0], pR = pr[3];
-  const double unL = fma(pl[1], nx, pl[2] * ny), unR = fma(pr[1], nx, pr[2] * ny);
-  const double utL = fma(pl[2], nx, -(pl[1] * ny)), utR = fma(pr[2], nx, -(pr[1] * ny));
-  const double mL = rhoL * unL, mR = rhoR * unR, tL = rhoL * utL;
+                                                   double nx, double ny, double af, double* flux, double& wsa) {
+  const double rhoL = pl[0], uL = pl[1], vL = pl[2], pL = pl[3];
+  const double rhoR = pr[0], uR = pr[1], vR = pr[2], pR = pr[3];
+  const double unL = fma(uL, nx, vL * ny), unR = fma(uR, nx, vR * ny);
+  const double utL = fma(vL, nx, -(uL * ny)), utR = fma(vR, nx, -(uR * ny));
+  const double mL = rhoL * unL, mR = rhoR * unR;
   // 2 rho H
-  const double EL = fma(mL, unL, fma(tL, utL, c2 * pL));
-  const double ER = fma(mR, unR, fma(rhoR * utR, utR, c2 * pR));
+  const double EL = fma(rhoL, fma(uL, uL, vL * vL), c2 * pL);
+  const double ER = fma(rhoR, fma(uR, uR, vR * vR), c2 * pR);
   const double g = rhoL * rhoR, rg = rsqrt_nr(g);
   const double rho = g * rg;
   const double w = rcp_nr(rhoL + rho);
-  const double un = fma(rho, unR, mL) * w, ut = fma(rho, utR, tL) * w;
+  const double un = fma(rho, unR, mL) * w, ut = fma(rho, utR, rhoL * utL) * w;
   const double H2 = fma(rhoL * rg, ER, EL) * w;  // 2 H
   const double q2 = fma(un, un, ut * ut);        // un^2 + ut^2
   const double a2 = hgm1 * (H2 - q2);
@@ -515,23 +515,18 @@ __device__ __forceinline__ void roe_flux_area_fp64(double hgm1, double c2, const
   const double ws1 = fabs(un);
   const double w1 = ws1 * (rho * (utR - utL)), w2 = ws1 * ((rhoR - rhoL) - A);
   const double s03 = scale2<-1>(w0 + w3), sd = s03 + w2, dw = (w3 - w0) * a;
-  const double Fn = fma(-0.5, dw, fma(-un, sd, fma(mL, unL, fma(mR, unR, pL + pR))));
-  const double Ft = fma(-ut, sd, fma(mL, utL, mR * utR)) - w1;
+  // dissipation of the normal and tangential momentum
+  const double Dn = fma(un, sd, scale2<-1>(dw)), Dt = fma(ut, sd, w1);
+  const double D1 = fma(Dn, nx, -(Dt * ny)), D2 = fma(Dn, ny, Dt * nx);
   const double D3 = fma(H2, s03, fma(scale2<1>(w1), ut, fma(un, dw, w2 * q2)));
-  const double hy = ny * s.h;
-  flux[0] = ((mL + mR) - sd) * s.h;
-  flux[1] = fma(Fn, s.hx, -(Ft * hy));
-  flux[2] = fma(Fn, hy, Ft * s.hx);
-  flux[3] = scale2<-1>((fma(unL, EL, unR * ER) - D3) * s.h);
-  wsa = (ws1 + a) * s.h;
+  const double pLR = pL + pR, h = scale2<-1>(af);
+  flux[0] = ((mL + mR) - sd) * h;
+  // (the smallest terms first: the pressure is the largest below Mach 1)
+  flux[1] = fma(pLR, nx, fma(mL, uL, fma(mR, uR, -D1))) * h;
+  flux[2] = fma(pLR, ny, fma(mL, vL, fma(mR, vR, -D2))) * h;
+  flux[3] = scale2<-1>((fma(unL, EL, unR * ER) - D3) * h);
+  wsa = (ws1 + a) * h;
 }
-__device__ __forceinline__ Area ld_area(const DevView& d, int e) {
-  const double2 a = reinterpret_cast<const double2*>(d.efac)[e];
-  return {a.x, a.y};
-}
-#else
-using Area = T;  // the face's length
-__device__ __forceinline__ Area ld_area(const DevView& d, int e) { return static_cast<const T*>(d.earea)[e]; }
 #endif
 
 // ---------------------------------------------------------------------------
@@ -967,7 +962,7 @@ __device__ __forceinline__ void roe_flux_area_df(df64 gm1, df64 ggm1, const df64
 
 // Roe flux of one edge slot from its face states, times the face length
 // (flux) and the wave speed times the length (wsa)
-__device__ __forceinline__ void flux_eval(const DevView& d, const T* pfL, const T* pfR, T2 n, Area af, T* flux,
+__device__ __forceinline__ void flux_eval(const DevView& d, const T* pfL, const T* pfR, T2 n, T af, T* flux,
                                           T& wsa) {
 #if FVS_FP64_FAST
   roe_flux_area_fp64(d.hgm1, d.c2, pfL, pfR, n.x, n.y, af, flux, wsa);
@@ -987,7 +982,7 @@ __device__ __forceinline__ void flux_eval(const DevView& d, const T* pfL, const 
 }
 
 // ... into the slot's record
-__device__ __forceinline__ void flux_finish(const DevView& d, int e, const T* pfL, const T* pfR, T2 n, Area af) {
+__device__ __forceinline__ void flux_finish(const DevView& d, int e, const T* pfL, const T* pfR, T2 n, T af) {
   T flux[4], wsa;
   flux_eval(d, pfL, pfR, n, af, flux, wsa);
   st4(static_cast<T*>(d.eflux), e, flux);
@@ -1100,14 +1095,14 @@ template <int REC, bool COH>
 struct FluxItem {
   int2 lr;
   T2 n, dl, dr;
-  Area af;
+  T af;
 
   __device__ __forceinline__ void load_static(const DevView& d, int e) {
     lr = d.ecell[e];
     lr.x = chk_idx(d.bounds_err, lr.x, 0, d.nc, SITE_EDGE_L);
     lr.y = chk_idx(d.bounds_err, lr.y, -1, d.nc, SITE_EDGE_R);
     n = ld2(d.enrm, e);
-    af = ld_area(d, e);
+    af = static_cast<const T*>(d.earea)[e];
     dl = {T(0), T(0)};
     dr = {T(0), T(0)};
     if (REC != REC_FIRST) {
@@ -1171,13 +1166,12 @@ __device__ __forceinline__ void flux_first_pair(const DevView& d, int e0, int e1
   const int e[2] = {e0, e1 >= 0 ? e1 : e0};
   int2 lr[2];
   T2 n[2];
-  Area af[2];
-  T pl[2][4], pr[2][4];
+  T af[2], pl[2][4], pr[2][4];
 #pragma unroll
   for (int j = 0; j < 2; j++) {
     lr[j] = d.ecell[e[j]];
     n[j] = ld2(d.enrm, e[j]);
-    af[j] = ld_area(d, e[j]);
+    af[j] = static_cast<const T*>(d.earea)[e[j]];
   }
 #pragma unroll
   for (int j = 0; j < 2; j++) {

@@ -14,7 +14,6 @@
 #include <cmath>
 #include <numeric>
 #include <string>
-#include <type_traits>
 #include <vector>
 
 #include "fvs_internal.hpp"
@@ -346,18 +345,6 @@ bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weig
   if (ok && csr) {
     ok = A.upload(dsp, L.st_ptr) && A.upload(t_coef, L.st_coef) && A.upload(dsn, L.st_node) && A.upload(t_ce, L.coefedg);
     d.st_ptr = dsp; d.st_coef = t_coef; d.st_node = dsn; d.coefedg = t_ce;
-  }
-  if (ok && std::is_same<T, double>::value && !weights) {
-    // FP64 kernels: the flux's factors of a face
-    std::vector<double> fac(2 * (size_t)L.ne);
-    for (size_t e = 0; e < (size_t)L.ne; e++) {
-      const double h = 0.5 * double(L.earea[e]);
-      fac[2 * e] = double(L.enrm[2 * e]) * h;
-      fac[2 * e + 1] = h;
-    }
-    double* p = nullptr;
-    ok = A.upload(p, fac);
-    d.efac = p;
   }
   if (!ok) return false;
   d.nc = L.nc;
