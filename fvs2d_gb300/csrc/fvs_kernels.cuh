@@ -458,7 +458,9 @@ __device__ __forceinline__ void roe_flux_fast(T gamma, T gm1, T igm1, const T* p
 //    the averaged density is sqrt(g), the weights rhoL and sqrt(g), and one
 //    reciprocal of their sum serves all three averages; rho H enters as
 //    2 rho H = rho (u^2 + v^2) + 2 gamma/(gamma-1) p, so no state's own
-//    density is divided by
+//    density is divided by.  Densities whose product leaves the range (below
+//    1e-154, above 1e154) take their ratio instead, behind a branch; two negative
+//    densities average to a negative one, as in the source form
 //  - reciprocals and square roots from the hardware approximations refined by
 //    one Newton-Raphson step (fp64_fast.cuh): 1/sqrt(g), 1/(rhoL + sqrt(g)) and
 //    1/sqrt(a^2), which gives a, 1/a and 1/a^2
@@ -500,11 +502,20 @@ __device__ __forceinline__ void roe_flux_area_fp64(double hgm1, double c2, const
   // 2 rho H
   const double EL = fma(rhoL, fma(uL, uL, vL * vL), c2 * pL);
   const double ER = fma(rhoR, fma(uR, uR, vR * vR), c2 * pR);
-  const double g = rhoL * rhoR, rg = rsqrt_nr(g);
-  const double rho = g * rg;
+  // averaged density sqrt(g), of the sign of the two, and rhoL over it
+  const double g = rhoL * rhoR;
+  const double rg = copysign(rsqrt_nr(g), rhoL);
+  double rho = g * rg, rl = rhoL * rg;
+  if (__builtin_expect((unsigned)((__double2hiint(g) >> 20 & 0x7ff) - 1) >= 0x7feu, 0)) {
+    // the product left the range of normal numbers: from the ratio
+    asm volatile("");
+    const double RT = sqrt_nr(rhoR * rcp_nr(rhoL));
+    rho = RT * rhoL;
+    rl = rcp_nr(RT);
+  }
   const double w = rcp_nr(rhoL + rho);
   const double un = fma(rho, unR, mL) * w, ut = fma(rho, utR, rhoL * utL) * w;
-  const double H2 = fma(rhoL * rg, ER, EL) * w;  // 2 H
+  const double H2 = fma(rl, ER, EL) * w;   // 2 H
   const double q2 = fma(un, un, ut * ut);        // un^2 + ut^2
   const double a2 = hgm1 * (H2 - q2);
   const double ra = rsqrt_nr(a2);
