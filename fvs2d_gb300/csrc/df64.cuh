@@ -98,23 +98,34 @@ __device__ __forceinline__ df64 dsqrt_(df64 x) {
   const float r = ((x.hi - p.hi) - p.lo) + x.lo;
   return fast_two_sum(s, __fdiv_rn(r, 2.0f * s));
 }
-// 1 / x and 1 / sqrt(x) of positive normal numbers: the FP32 approximation y
-// corrected by its residual e, formed in one or two exact products: y (1 + e +
-// e^2) with e = 1 - x y, and y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2 (the
-// series forms of fp64_fast.cuh).  |e| < 2^-21, so what is left out lies below
-// 2^-63 and the correction, rounded to FP32, is exact to 2^-45 of the result or better.
-__device__ __forceinline__ df64 drcp_(df64 x) {
+// 1 / x: the FP32 reciprocal y corrected by its residual e = 1 - x y, exact but
+// for the rounding of its low part: y (1 + e + e^2).  |e| <= 2^-23, so what is left out
+// lies below 2^-69.  Relative error at most 2^-46.4, root mean square 2^-49.1 (the
+// division operator: 2^-46.2, 2^-49.1; tests/test_df64_host.py).
+__host__ __device__ __forceinline__ df64 drcp_(df64 x) {
+#ifdef __CUDA_ARCH__
   const float y = __frcp_rn(x.hi);
-  const float e = __fmaf_rn(-x.lo, y, __fmaf_rn(-x.hi, y, 1.0f));
-  return fast_two_sum(y, y * __fmaf_rn(e, e, e));
+#else
+  const float y = 1.0f / x.hi;
+#endif
+  const float e = fmaf(-x.lo, y, fmaf(-x.hi, y, 1.0f));
+  return fast_two_sum(y, y * fmaf(e, e, e));
 }
-__device__ __forceinline__ df64 drsqrt_(df64 x) {
-  const float y = rsqrtf(x.hi);
-  const df64 p = two_prod(y, y);
-  const df64 q = two_prod(x.hi, p.hi);  // q + the terms below: x y^2
-  const float e = (1.0f - q.hi) - (q.lo + __fmaf_rn(x.hi, p.lo, x.lo * p.hi));
-  return fast_two_sum(y, y * e * __fmaf_rn(0.375f, e, 0.5f));
+// sqrt(x) of a positive normal number from an approximation y of 1 / sqrt(x.hi)
+// a few units off: s, the FP32 root rounded to nearest by one Newton step, and
+// its exact residual over 2 s, that quotient corrected once more.  As exact as
+// dsqrt_ (at most 2^-46.4, root mean square 2^-49.5, for any y within 2 units)
+// without its IEEE root and division.  A reciprocal root y (1 + e / 2 + 3 e^2 / 8)
+// instead carries the rounding of a correction of up to 2^-22: 2^-44, 2^-47.1.
+__host__ __device__ __forceinline__ df64 dsqrt_from(df64 x, float y) {
+  const float h = 0.5f * y, s0 = x.hi * y;
+  const float s = fmaf(h, fmaf(-s0, s0, x.hi), s0);
+  const df64 p = two_prod(s, s);
+  const float r = ((x.hi - p.hi) - p.lo) + x.lo;
+  const float c = r * h;
+  return fast_two_sum(s, fmaf(fmaf(-2.0f * s, c, r), h, c));
 }
+__device__ __forceinline__ df64 dsqrt_pos(df64 x) { return dsqrt_from(x, rsqrtf(x.hi)); }
 // a + b, sloppy: one TwoSum of the high parts, the low parts added to its
 // error, renormalised
 __device__ __forceinline__ df64 dadd_s(df64 a, df64 b) {

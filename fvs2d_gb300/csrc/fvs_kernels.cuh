@@ -925,10 +925,10 @@ enum : int { REC_GENERAL = 0, REC_SPEC = 1, REC_FIRST = 2 };
 // the densities (their product leaves FP32's range sooner); every FP64 fused
 // multiply-add there is dfma here and the sums of like-signed terms are
 // sloppy sums (df64.cuh), while the differences of face values, wave speeds
-// and dissipation terms keep the accurate sum.  The two reciprocals and two
-// reciprocal square roots are FP32 approximations corrected by their exact
-// residual (drcp_, drsqrt_), where the form with x and y velocities took four
-// divisions and two roots.  Its error stays near 2^-47 of the flux's operands.
+// and dissipation terms keep the accurate sum.  The four reciprocals and two
+// square roots are FP32 approximations corrected by their exact residual
+// (drcp_, dsqrt_pos), where the form with x and y velocities took four divisions
+// and two roots.
 // (SSP-RK3 step of 1,048,576 cells: 509 -> 479 us.)
 __device__ __forceinline__ df64 harten(df64 x) {
   const df64 w = dabs_(x);
@@ -944,20 +944,18 @@ __device__ __forceinline__ void roe_flux_area_df(df64 gm1, df64 ggm1, const df64
   // 2 rho H
   const df64 EL = dfma(mL, unL, dfma(tL, utL, c2 * pL));
   const df64 ER = dfma(mR, unR, dfma(rhoR * utR, utR, c2 * pR));
-  const df64 riL = drcp_(rhoL), x = rhoR * riL, rx = drsqrt_(x), RT = x * rx;
+  const df64 RT = dsqrt_pos(rhoR * drcp_(rhoL)), rx = drcp_(RT);
   const df64 rho = RT * rhoL;
-  const df64 w = riL * drcp_(dadd_s(df64(1.f, 0.f), RT));
+  const df64 w = drcp_(dadd_s(rhoL, rho));
   const df64 un = dfma(rho, unR, mL) * w, ut = dfma(rho, utR, tL) * w;
   const df64 H2 = dfma(rx, ER, EL) * w;   // 2 H
   const df64 q2 = dfma(un, un, ut * ut);        // un^2 + ut^2
   const df64 a2 = half(gm1) * (H2 - q2);
-  const df64 ra = drsqrt_(a2);
-  const df64 a = a2 * ra;
-  const df64 dp = pR - pL;
-  const df64 A = dp * (ra * ra), B = rho * (unR - unL) * ra;
-  const df64 w0 = harten(un - a) * (A - B), w3 = harten(un + a) * (A + B);  // twice the strengths
+  const df64 a = dsqrt_pos(a2), ia2 = drcp_(a2);
+  const df64 dp = pR - pL, rad = rho * a * (unR - unL);
+  const df64 w0 = harten(un - a) * ((dp - rad) * ia2), w3 = harten(un + a) * ((dp + rad) * ia2);  // twice the strengths
   const df64 ws1 = dabs_(un);
-  const df64 w1 = ws1 * (rho * (utR - utL)), w2 = ws1 * ((rhoR - rhoL) - A);
+  const df64 w1 = ws1 * (rho * (utR - utL)), w2 = ws1 * dfma(-dp, ia2, rhoR - rhoL);
   const df64 s03 = half(w0 + w3), sd = s03 + w2, hdw = half((w3 - w0) * a);
   const df64 haf = half(af), hx = nx * haf, hy = ny * haf;
   const df64 Fn = dfma(-un, sd, dfma(mL, unL, dfma(mR, unR, dadd_s(pL, pR)))) - hdw;
