@@ -3,15 +3,22 @@ residuals and wave-speed sums against extended precision.
 
 The states keep the conversion to primitives exact (density 1, velocities and
 pressure multiples of 2^-12, gamma 3/2), so that what is measured is the flux
-and its sum over the faces.  Bar: the FP64 momentum no
-further off than the strict mode's, which takes the source's order (an
-emulation of both gives 0.71 to 0.83 of it; 1.12 to 1.29 when the momentum flux
-is turned back from the face's frame as a whole)."""
+and its sum over the faces.  Bars, in units of pressure times the mean face
+length for the momentum and relative for the wave speed:
+
+FP64: the momentum no further off than the strict mode's, which takes the
+source's order (an emulation of both gives 0.71 to 0.83 of it; 1.12 to 1.29
+when the momentum flux is turned back from the face's frame as a whole).
+
+Double-float, log2: emulated with the correctly rounded roots and divisions
+and the momentum summed in x and y -48.1 (Mach 0.01) and -47.9 (0.5) for the
+momentum, -49.0 and -49.1 for the wave speed; turned back from the face's frame
+with a reciprocal root of 2^-44, 0.5 and 1.1 to 0.9 more.  Half way."""
 import numpy as np
 import pytest
 
 import cases
-from fvs2d_gb300 import PREC_FP64, PREC_FP64_STRICT, Solver
+from fvs2d_gb300 import PREC_FP64, PREC_FP64_DF, PREC_FP64_STRICT, Solver
 
 pytestmark = pytest.mark.gpu
 
@@ -78,3 +85,9 @@ def test_fp64_momentum(mach):
     e = errors(mach, (PREC_FP64_STRICT, PREC_FP64))
     assert e[PREC_FP64_STRICT][0] < 1e-14  # the extended-precision residual is the strict mode's
     assert e[PREC_FP64][0] <= e[PREC_FP64_STRICT][0], (e, e[PREC_FP64][0] / e[PREC_FP64_STRICT][0])
+
+
+@pytest.mark.parametrize("mach,momentum,wave", [(0.01, -47.85, -48.5), (0.5, -47.65, -48.6)])
+def test_double_float(mach, momentum, wave):
+    m, w = errors(mach, (PREC_FP64_DF,))[PREC_FP64_DF]
+    assert np.log2(m) <= momentum and np.log2(w) <= wave, (np.log2(m), np.log2(w))
