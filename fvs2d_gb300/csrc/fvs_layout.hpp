@@ -39,12 +39,14 @@ struct DeviceArena {
     dst = static_cast<V*>(p);
     return true;
   }
-  bool alloc(void*& dst, size_t bytes) {
+  // zeroed when the call returns; wait = false: when the next upload has returned
+  // (both are in the order of the legacy stream)
+  bool alloc(void*& dst, size_t bytes, bool wait = true) {
     dst = nullptr;
     if (bytes == 0) bytes = 16;
     if (cudaMalloc(&dst, bytes) != cudaSuccess) return false;
     allocs.push_back(dst);
-    return zero_sync(dst, bytes) == cudaSuccess;
+    return (wait ? zero_sync(dst, bytes) : cudaMemsetAsync(dst, 0, bytes, nullptr)) == cudaSuccess;
   }
 };
 
@@ -358,7 +360,9 @@ bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weig
   return true;
 }
 
-// Allocates the state and work arrays of a view with nc cells, ne edges.
+// Allocates the state and work arrays of a view with nc cells, ne edges; they
+// are zero once a later upload of the same thread has returned (its callers
+// upload phi next).
 template <typename T>
 bool alloc_work(DeviceArena& A, DevView& d, int nc, int ne, int nblk, int norm_cap) {
   void* p;
@@ -367,7 +371,7 @@ bool alloc_work(DeviceArena& A, DevView& d, int nc, int ne, int nblk, int norm_c
   d.nblk_red = nblk;
   d.norm_cap = norm_cap;
 #define FVS_ALLOC(field, type, bytes) \
-  ok = ok && A.alloc(p, bytes);       \
+  ok = ok && A.alloc(p, bytes, false); \
   d.field = static_cast<type>(p)
   FVS_ALLOC(U, double*, 8 * n4);
   FVS_ALLOC(U0, double*, 8 * n4);
