@@ -134,11 +134,26 @@ __device__ __forceinline__ df64 dadd_s(df64 a, df64 b) {
 }
 // a * b + c: TwoProd of the high parts, TwoSum with c's high part, the
 // cross terms and both low parts in one FP32 sum, renormalised
-__device__ __forceinline__ df64 dfma(df64 a, df64 b, df64 c) {
+__host__ __device__ __forceinline__ df64 dfma(df64 a, df64 b, df64 c) {
   const df64 p = two_prod(a.hi, b.hi);
-  const float cross = __fmaf_rn(a.hi, b.lo, a.lo * b.hi);
+  const float cross = fmaf(a.hi, b.lo, a.lo * b.hi);
   const df64 s = two_sum(p.hi, c.hi);
   return fast_two_sum(s.hi, s.lo + ((p.lo + cross) + c.lo));
+}
+// c + q and a * b + c for a c that outweighs the other term: the low parts that
+// matter, the high sum's error and c's, added exactly.  One rounding of 2^-49 of
+// c is left: root mean square 2^-49.95 of a face value p + phi (...), where a
+// product and the accurate sum give 2^-49.7, dfma 2^-49.6 and two in a chain
+// 2^-49.1 (tests/test_df64_host.py); 18 and 22 instructions.
+__host__ __device__ __forceinline__ df64 dadd_big(df64 c, df64 q) {
+  const df64 s = two_sum(c.hi, q.hi);
+  const df64 t = two_sum(s.lo, c.lo);
+  return fast_two_sum(s.hi, t.hi + (t.lo + q.lo));
+}
+__host__ __device__ __forceinline__ df64 dfma_big(df64 a, df64 b, df64 c) {
+  df64 p = two_prod(a.hi, b.hi);
+  p.lo += fmaf(a.hi, b.lo, a.lo * b.hi);
+  return dadd_big(c, p);
 }
 __device__ __forceinline__ df64 dabs_(df64 x) { return x.hi < 0.0f ? -x : x; }
 __device__ __forceinline__ df64 half(df64 x) { return df64(0.5f * x.hi, 0.5f * x.lo); }

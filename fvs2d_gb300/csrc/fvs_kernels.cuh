@@ -1046,8 +1046,8 @@ __device__ __forceinline__ void face_states(const DevView& d, int e, bool interi
 #pragma unroll
         for (int v = 0; v < 4; v++) {
 #if FVS_DF
-          pfL[v] = dfma(phiL, dfma(dl.x, gxl[v], dl.y * gyl[v]), pl[v]);
-          pfR[v] = dfma(phiR, dfma(dr.x, gxr[v], dr.y * gyr[v]), pr[v]);
+          pfL[v] = dfma_big(phiL, dfma(dl.x, gxl[v], dl.y * gyl[v]), pl[v]);
+          pfR[v] = dfma_big(phiR, dfma(dr.x, gxr[v], dr.y * gyr[v]), pr[v]);
 #else
           pfL[v] = fma(phiL, fma(dl.x, gxl[v], dl.y * gyl[v]), pl[v]);
           pfR[v] = fma(phiR, fma(dr.x, gxr[v], dr.y * gyr[v]), pr[v]);
@@ -1068,12 +1068,13 @@ __device__ __forceinline__ void face_states(const DevView& d, int e, bool interi
 #elif FVS_DF
         const T gradL = dfma(dl.x, gxl[v], dl.y * gyl[v]);
         const T gradR = dfma(dr.x, gxr[v], dr.y * gyr[v]);
+        const T stepL = dfma(kh, gradC, omk * gradL), stepR = dfma(nkh, gradC, omk * gradR);
         if (d.limiter == FVS_LIM_NONE) {  // phi = 1
-          pfL[v] = dfma(kh, gradC, dfma(omk, gradL, pl[v]));
-          pfR[v] = dfma(nkh, gradC, dfma(omk, gradR, pr[v]));
+          pfL[v] = dadd_big(pl[v], stepL);
+          pfR[v] = dadd_big(pr[v], stepR);
         } else {
-          pfL[v] = dfma(phiL, dfma(kh, gradC, omk * gradL), pl[v]);
-          pfR[v] = dfma(phiR, dfma(nkh, gradC, omk * gradR), pr[v]);
+          pfL[v] = dfma_big(phiL, stepL, pl[v]);
+          pfR[v] = dfma_big(phiR, stepR, pr[v]);
         }
 #else
         const T gradL = dl.x * gxl[v] + dl.y * gyl[v];
