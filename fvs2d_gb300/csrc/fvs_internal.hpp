@@ -121,9 +121,9 @@ struct DevView {
   const void* cpos = nullptr;    // [nc][4] x 2 face-centre offsets (T) for the limiter
   const int8_t* nvrt = nullptr;
   // gradient stencil interleaved over groups of 32 cells: entry j of cell ic
-  // at ell_base[ic / 32] + 32 j + ic % 32, j < ell_n[ic]
-  const int* ell_base = nullptr;
-  const uint16_t* ell_n = nullptr;
+  // at 32 (ell_row[ic / 32] + j) + ic % 32, j < ell_n[ic]
+  const int* ell_row = nullptr;
+  const int* ell_n = nullptr;
   int st_max = 0;                  // longest stencil
   const int* ell_cell = nullptr;
   const void* ell_coef = nullptr;  // x 2 (T); GGNB: edge times node coefficient

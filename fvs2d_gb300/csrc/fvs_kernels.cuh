@@ -737,16 +737,19 @@ struct StencilChunk {
 #if FVS_STRICT
   T w[CH];
 #endif
-  // entries [j0, j0 + CH) below n; at: the cell's place of entry 0
-  __device__ __forceinline__ void load(const DevView& d, int at, int j0, int n) {
+  // the first CH of the n entries from place `at` on.  (Places are counted in
+  // 64 bits: rows padded to their group's longest stencil can pass 2^31 places
+  // where the stencils' own entries do not.)
+  __device__ __forceinline__ void load(const DevView& d, size_t at, int n) {
+    const int* cell = d.ell_cell + at;
+    const T2* coef = static_cast<const T2*>(d.ell_coef) + at;
 #pragma unroll
     for (int q = 0; q < CH; q++) {
-      const int k = at + 32 * (j0 + q);
-      if (j0 + q < n) {
-        id[q] = chk_idx(d.bounds_err, d.ell_cell[k], 0, d.nc, SITE_STENCIL);
-        c[q] = ld2(d.ell_coef, k);
+      if (q < n) {
+        id[q] = chk_idx(d.bounds_err, cell[32 * q], 0, d.nc, SITE_STENCIL);
+        c[q] = coef[32 * q];
 #if FVS_STRICT
-        w[q] = d.ell_w ? static_cast<const T*>(d.ell_w)[k] : T(1);
+        w[q] = d.ell_w ? static_cast<const T*>(d.ell_w)[at + 32 * q] : T(1);
 #endif
       }
     }
@@ -758,15 +761,16 @@ struct StencilChunk {
 // the primitives.
 template <int METHOD, int LIM, bool COH, int CH>
 struct GradientItem {
-  int at, n;
+  size_t at;
+  int n;
   T2 c0;
   StencilChunk<CH> ch;
 
   __device__ __forceinline__ void load_static(const DevView& d, int ic) {
-    at = d.ell_base[ic >> 5] + (ic & 31);
+    at = 32 * (size_t)d.ell_row[ic >> 5] + (ic & 31);
     n = d.ell_n[ic];
     c0 = own_coef<METHOD>(d, ic);
-    ch.load(d, at, 0, n);
+    ch.load(d, at, n);
   }
   __device__ __forceinline__ void run(const DevView& d, int ic) {
     const T* P = static_cast<const T*>(d.Pv);
@@ -790,7 +794,7 @@ struct GradientItem {
         }
       j0 += CH;
       if (j0 >= n) break;
-      ch.load(d, at, j0, n);
+      ch.load(d, at + 32 * (size_t)j0, n - j0);
     }
     T ph;
     s.finish(d, ic, pc, ph);

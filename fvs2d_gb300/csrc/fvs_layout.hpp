@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <new>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -135,47 +136,49 @@ struct Layout {
   std::vector<int8_t> st_node;
   // the stencil interleaved over groups of 32 cells (build_ell): per group as
   // many rows of 32 entries as its longest stencil has
-  std::vector<int> ell_base, ell_cell;
-  std::vector<uint16_t> ell_n;  // (a stencil of n cells around one node occurs n times: 65,535 is beyond any 32-bit total)
+  std::vector<int> ell_row, ell_n, ell_cell;
   std::vector<T> ell_coef, ell_w;
 
-  // from the CSR rows, entry order kept; places beyond a cell's own entries
-  // hold cell 0 and zeros and are not read
-  bool build_ell() {
-    const int ng = (nc + 31) / 32;
-    const bool node = !st_node.empty();
-    ell_base.assign(1, 0);
+  // rows before every group, and the stencils' lengths, from the CSR rows.  A
+  // row holds an entry of its own, so the rows fit the 32 bits that the CSR
+  // entries are counted in; the places, 32 per row, need not.
+  void build_ell_rows() {
+    ell_row.assign(1, 0);
     ell_n.resize(nc);
-    long long total = 0;
-    for (int g = 0; g < ng; g++) {
+    for (int g = 0; g < nc; g += 32) {
       int width = 0;
-      for (int ic = 32 * g; ic < std::min(nc, 32 * g + 32); ic++) {
-        const int n = st_ptr[ic + 1] - st_ptr[ic];
-        if (n > 65535) return false;
-        ell_n[ic] = (uint16_t)n;
-        width = std::max(width, n);
+      for (int ic = g; ic < std::min(nc, g + 32); ic++) {
+        ell_n[ic] = st_ptr[ic + 1] - st_ptr[ic];
+        width = std::max(width, ell_n[ic]);
       }
-      total += 32LL * width;
-      if (total > 0x7fffffffLL) return false;
-      ell_base.push_back((int)total);
+      ell_row.push_back(ell_row.back() + width);
     }
-    ell_cell.assign((size_t)total, 0);
-    ell_coef.assign(2 * (size_t)total, T(0));
-    if (!st_w.empty()) ell_w.assign((size_t)total, T(0));
+  }
+  size_t ell_place(int ic, int j) const { return 32 * (size_t)(ell_row[ic / 32] + j) + ic % 32; }
+
+  // entry order kept; places beyond a cell's own entries hold cell 0 and zeros
+  // and are not read
+  void build_ell() {
+    build_ell_rows();
+    const bool node = !st_node.empty();
+    const size_t total = 32 * (size_t)ell_row.back();
+    ell_cell.assign(total, 0);
+    ell_coef.assign(2 * total, T(0));
+    if (!st_w.empty()) ell_w.assign(total, T(0));
     for (int ic = 0; ic < nc; ic++)
-      for (int k = st_ptr[ic], at = ell_base[ic / 32] + ic % 32; k < st_ptr[ic + 1]; k++, at += 32) {
+      for (int k = st_ptr[ic]; k < st_ptr[ic + 1]; k++) {
+        const size_t at = ell_place(ic, k - st_ptr[ic]);
         ell_cell[at] = st_cell[k];
         if (node) {
           const T* ce = &coefedg[8 * (size_t)ic + 2 * st_node[k]];
-          ell_coef[2 * (size_t)at] = ce[0] * st_coef[k];
-          ell_coef[2 * (size_t)at + 1] = ce[1] * st_coef[k];
+          ell_coef[2 * at] = ce[0] * st_coef[k];
+          ell_coef[2 * at + 1] = ce[1] * st_coef[k];
         } else {
-          ell_coef[2 * (size_t)at] = st_coef[2 * (size_t)k];
-          ell_coef[2 * (size_t)at + 1] = st_coef[2 * (size_t)k + 1];
+          ell_coef[2 * at] = st_coef[2 * (size_t)k];
+          ell_coef[2 * at + 1] = st_coef[2 * (size_t)k + 1];
         }
         if (!st_w.empty()) ell_w[at] = st_w[k];
       }
-    return true;
   }
 };
 
@@ -328,17 +331,20 @@ int append_case(Layout<T>& L, const HostMesh& h, bool fold_w, int cs, std::strin
 // weights (the strict kernels read them).
 template <typename T>
 bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weights) {
-  if (!L.build_ell()) return false;
+  try {
+    L.build_ell();
+  } catch (const std::bad_alloc&) {
+    return false;
+  }
   bool ok = true;
   double *dvol, *drvol;
   int4* dcf;
   int8_t *dnv, *dsn;
-  int *dsp, *deb, *d_eb, *d_ec;
-  uint16_t* d_en;
+  int *dsp, *deb, *d_er, *d_en, *d_ec;
   int2* dec;
   T *t_rvol, *t_eps2, *t_cpos, *t_coef, *t_w = nullptr, *t_c0, *t_ce, *t_ell, *t_nrm, *t_area, *t_edL, *t_edR, *t_exy;
   ok = ok && A.upload(dvol, L.vol) && A.upload(drvol, L.rvol) && A.upload(dcf, L.cf) && A.upload(dnv, L.nvrt);
-  ok = ok && A.upload(d_eb, L.ell_base) && A.upload(d_en, L.ell_n) && A.upload(d_ec, L.ell_cell) && A.upload(t_ell, L.ell_coef);
+  ok = ok && A.upload(d_er, L.ell_row) && A.upload(d_en, L.ell_n) && A.upload(d_ec, L.ell_cell) && A.upload(t_ell, L.ell_coef);
   ok = ok && A.upload(dec, L.ecell);
   ok = ok && A.upload(deb, L.ebtype) && A.upload(t_rvol, L.rvolT) && A.upload(t_eps2, L.eps2);
   ok = ok && A.upload(t_cpos, L.cpos) && (!weights || A.upload(t_w, L.ell_w));
@@ -354,7 +360,7 @@ bool upload_layout(DeviceArena& A, Layout<T>& L, DevView& d, bool csr, bool weig
   d.nedge = L.ne;
   d.vol = dvol; d.rvol = drvol; d.cflist = dcf; d.nvrt = dnv;
   d.st_max = L.ell_n.empty() ? 0 : *std::max_element(L.ell_n.begin(), L.ell_n.end());
-  d.ell_base = d_eb; d.ell_n = d_en; d.ell_cell = d_ec; d.ell_coef = t_ell; d.ell_w = t_w;
+  d.ell_row = d_er; d.ell_n = d_en; d.ell_cell = d_ec; d.ell_coef = t_ell; d.ell_w = t_w;
   d.ecell = dec; d.ebtype = deb; d.volT = t_rvol; d.eps2 = t_eps2; d.cpos = t_cpos;
   d.coef0 = t_c0; d.enrm = t_nrm; d.earea = t_area; d.edL = t_edL; d.edR = t_edR; d.exy = t_exy;
   return true;
