@@ -210,6 +210,7 @@ void init_view_constants(fvs_batch* B, DevView& d) {
   d.ggm1 = ob.gamma / (ob.gamma - 1.0);
   d.khalf = ob.umuscl / 2.0; d.nkhalf = -ob.umuscl / 2.0; d.omk = 1.0 - ob.umuscl; d.cfl = ob.cfl;
   set_constants(d);
+  d.nsm = B->nsm;
   d.limiter = ob.limiter; d.grad_method = ob.grad_method; d.first_order = ob.reconst == FVS_RECON_UPWIND1;
   d.vortex = ob.vortex; d.vx = ob.vortex_x; d.vy = ob.vortex_y; d.vkappa = ob.vortex_kappa;
   for (int k = 0; k < 4; k++) { d.vinf[k] = ob.vortex_inf[k]; d.pinf[k] = B->pinf[k]; }
@@ -621,7 +622,7 @@ int fvs_batch_create(const fvs_mesh* meshes, const fvs_options* opts, int32_t nc
   cudaEventCreate(&B->ev1);
   cudaEventCreate(&B->eva);
   cudaEventCreate(&B->evb);
-  cudaDeviceGetAttribute(&B->nsm, cudaDevAttrMultiProcessorCount, 0);
+  B->nsm = sm_count();
   init_view_constants(B.get(), B->d);
   int rc = build_for(B.get(), B->prec, B->d);
   if (!rc) rc = alloc_batch_buffers(B.get());

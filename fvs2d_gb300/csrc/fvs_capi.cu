@@ -660,6 +660,7 @@ int fvs_create(const fvs_mesh* mesh, const fvs_options* opt, fvs_handle** out) {
   d.igm1 = 1.0 / (H->o.gamma - 1.0);
   d.ggm1 = H->o.gamma / (H->o.gamma - 1.0);
   set_constants(d);
+  d.nsm = sm_count();
   d.limiter = H->o.limiter;
   d.grad_method = H->o.grad_method;
   d.first_order = H->o.reconst == FVS_RECON_UPWIND1;

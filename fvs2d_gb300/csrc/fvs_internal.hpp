@@ -22,6 +22,15 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// streaming multiprocessors of the current device (152 on a whole GB300, whose
+// figures stand beside the launch rules)
+inline int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+    return 152;
+  return n;
+}
+
 // Host data, and zeros, in device memory when the call returns.  A cudaMemcpy
 // from pageable memory may return once its source is staged, and a cudaMemset
 // returns at once; the handles' streams are non-blocking, so their kernels are
@@ -151,6 +160,7 @@ struct DevView {
   int norm_cap = 0;
   int* bounds_err = nullptr;      // [4] index-checking kernels: flag, site, index, extent
   int* stepctl = nullptr;         // [0] = steps done in this call; right behind tctl (one upload sets both)
+  int nsm = 0;                    // multiprocessors of the device
   int trig_first = 0;             // the launch's pdl_trigger before its work (else after it)
   int upd_grid = 0;               // blocks of the last stage's update launch, which strides over the cells
                                   // (one wave of resident blocks; 0: one block per 256 cells)

@@ -84,7 +84,7 @@ __device__ __forceinline__ int chk_idx(int* err, int i, int lo, int hi, int site
 // runs and its mesh loads overlap with it, but they go to the SMs that have
 // room left, unevenly: a grid of less than a few waves then runs twice over on
 // some SMs.  So the step kernels call it before their work where the grid
-// leaves half of the 152 SMs free (SSP-RK3 step, before / after the work:
+// leaves half of the SMs free (152 SMs, SSP-RK3 step, before / after the work:
 // double-float 2,048 cells 34.8 / 45.1 us, 8,192 cells 42.9 / 44.9) and where it fills the chip for
 // several waves (mixed 524,000 cells 104.8 / 108.5 us, FP64 264,000 cells 449 / 458), and after it in between
 // (FP64 8,192 cells 89.5 / 49.1 us, 32,000 cells 155 / 84, 131,000 cells 262 /
@@ -3082,7 +3082,8 @@ static inline unsigned grid_of(int n) { return (unsigned)((n + 255) / 256); }
 // its pdl_trigger (see there)
 static DevView with_trigger(const DevView& d, unsigned grid, unsigned block) {
   DevView v = d;
-  v.trig_first = grid <= 76 || (unsigned long long)grid * block >= 200000;
+  // (several waves: 200,000 threads on 152 SMs)
+  v.trig_first = grid <= (unsigned)d.nsm / 2 || 152ull * grid * block >= 200000ull * d.nsm;
   return v;
 }
 static inline unsigned grid_for(int n, unsigned block) { return ((unsigned)n + block - 1) / block; }
@@ -3099,7 +3100,7 @@ static void launch_gradient_t(const DevView& d, cudaStream_t s) {
   const unsigned b = BLK_GRADIENT, g = grid_for(d.nc, b);
   // at most one block of 256 threads per SM, and stencils longer than the
   // other kernel's chunk
-  if (d.nc <= 152 * 256 && d.st_max > GRAD_CHUNK)
+  if (d.nc <= d.nsm * 256 && d.st_max > GRAD_CHUNK)
     launch_k(k_gradient<METHOD, LIM, true>, g, b, 0, s, with_trigger(d, g, b));
   else
     launch_k(k_gradient<METHOD, LIM, false>, g, b, 0, s, with_trigger(d, g, b));

@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "../../include/fvs2d.h"
+#include "fvs_internal.hpp"
 #include "fvs_tcgemm.cuh"
 
 namespace {
@@ -279,6 +280,7 @@ struct fvs_mlp {
   int* gemm_err = nullptr;           // set by a tcgen05 GEMM whose bounded wait expired
   int engine = 0;                    // 0: tcgen05, 1: mma.sync
   int step = 0;
+  int nsm = fvs::sm_count();             // multiprocessors of the device
   std::vector<void*> owned;
 
   ~fvs_mlp() {
@@ -352,9 +354,9 @@ template <bool A_KM, bool B_KM, int OUT>
 void gemm_tc(fvs_mlp* m, const tc::GemmArgs& a) {
   const long long rows = (a.M + tc::BM - 1) / tc::BM;
   if constexpr (wide_tiles(OUT)) {
-    if (a.N >= 128 && rows * ((a.N + 127) / 128) > 304) return gemm_tc_launch<A_KM, B_KM, OUT, 2, 128>(m, a);
+    if (a.N >= 128 && rows * ((a.N + 127) / 128) > 2 * m->nsm) return gemm_tc_launch<A_KM, B_KM, OUT, 2, 128>(m, a);
   }
-  if (rows * ((a.N + 63) / 64) > 304) gemm_tc_launch<A_KM, B_KM, OUT, 2, 64>(m, a);
+  if (rows * ((a.N + 63) / 64) > 2 * m->nsm) gemm_tc_launch<A_KM, B_KM, OUT, 2, 64>(m, a);
   else gemm_tc_launch<A_KM, B_KM, OUT, 4, 64>(m, a);
 }
 
@@ -427,12 +429,14 @@ void forward(fvs_mlp* m, int n, const float* y, const int* idx, float* pred) {
 }
 
 // The runs of K blocks that the parameter gradients are summed in (tc::k_grads).
-// A layer's runs are as many as make about one 128 x 128 tile per SM: their number
+// A layer's runs are as many as make GRAD_TILES tiles of 128 x 128: their number
 // fixes the order of the FP32 sums, and with it the training's trajectory (runs
 // five times longer, added in the same order, moved a weight by 5e-5 of the
 // weights' norm after 32 steps, through BF16 roundings that fell the other way).
+// So it is a constant, near the number of SMs but not bound to the device's.
 // A CTA takes as many consecutive runs as leave the launch in one wave of four
 // CTAs per SM.
+constexpr int GRAD_TILES = 148;
 bool grad_plan(fvs_mlp* m, int rows, tc::GradPlan& p) {
   p = tc::GradPlan();
   p.nl = m->nl;
@@ -449,7 +453,7 @@ bool grad_plan(fvs_mlp* m, int rows, tc::GradPlan& p) {
     const int square = ((g.din + 127) / 128) * ((g.dout + 127) / 128);
     g.per = nk;
     if (square < 64 && nk >= 4) {
-      const int want = std::max(1, 148 / square);
+      const int want = std::max(1, GRAD_TILES / square);
       g.per = std::max(1, (nk + want - 1) / want);
     }
     g.nsplit = (nk + g.per - 1) / g.per;
@@ -460,7 +464,7 @@ bool grad_plan(fvs_mlp* m, int rows, tc::GradPlan& p) {
   }
   int bias_ctas = 0;
   for (int l = 0; l < m->nl; l++) bias_ctas += (m->dout[l] + tc::BIAS_COLS - 1) / tc::BIAS_COLS;
-  const int room = std::max(304, 608 - bias_ctas);
+  const int room = std::max(2 * m->nsm, 4 * m->nsm - bias_ctas);
   p.runs = (int)std::max<long long>(1, (tile_runs + room - 1) / room);
   for (int l = 0; l < m->nl; l++) {
     tc::GradLayer& g = p.l[l];
