@@ -1218,11 +1218,15 @@ __device__ __forceinline__ void flux_range(const DevView& d, int b, int end, int
 
 #if FVS_FP64_FAST && !FVS_BOUNDS
 // The same flux with the Roe average in x and y velocities, from 1/rhoL,
-// 1/rhoR and 1/(1+RT): the base residual of a defect-correction chunk.  That
-// residual is rounded to FP32 near convergence, where it is what cancellation
-// leaves of the fluxes, and the iteration follows the last bits of what is
-// rounded (with the form above the reported increments moved by 2e-7); once
-// per chunk its 18 more operations per edge do not show.
+// 1/rhoR and 1/(1+RT): the base residual of a defect-correction chunk.  It is
+// not the more exact of the two: emulated against 128-bit arithmetic the form
+// above has 0.83 to 1.0 of its rounding error in the momentum and 0.92 to 1.0 in
+// the energy (jumps of 0.1 and 50 %, Mach 0.01 to 3).  It stays because near
+// convergence the residual, rounded to FP32, is what cancellation leaves of the
+// fluxes, so the increments that a run reports follow these last bits: with the
+// form above they move by 1e-7 to 3e-7 of their value after 400 steps (six
+// airfoils), and a run is to report what it reported.  Once per chunk its 17
+// more operations per edge cost 1 % (25.2 against 24.9 ms for the 400 steps).
 __device__ __forceinline__ void roe_flux_xy_fp64(double gm1, double ggm1, const double* pl, const double* pr,
                                                    double nx, double ny, double af, double* flux, double& wsa) {
   const double rhoL = pl[0], uL = pl[1], vL = pl[2], pL = pl[3];
