@@ -761,16 +761,18 @@ struct StencilChunk {
 // the primitives.
 template <int METHOD, int LIM, bool COH, int CH>
 struct GradientItem {
-  size_t at;
-  int n;
+  int row, n;
   T2 c0;
   StencilChunk<CH> ch;
 
+  // (the 64-bit place itself, kept, is spilled in double-float)
+  __device__ __forceinline__ size_t place(int ic, int j) const { return 32 * (size_t)(unsigned)(row + j) + (ic & 31); }
+
   __device__ __forceinline__ void load_static(const DevView& d, int ic) {
-    at = 32 * (size_t)d.ell_row[ic >> 5] + (ic & 31);
+    row = d.ell_row[ic >> 5];
     n = d.ell_n[ic];
     c0 = own_coef<METHOD>(d, ic);
-    ch.load(d, at, n);
+    ch.load(d, place(ic, 0), n);
   }
   __device__ __forceinline__ void run(const DevView& d, int ic) {
     const T* P = static_cast<const T*>(d.Pv);
@@ -778,23 +780,23 @@ struct GradientItem {
     ldc4<COH>(P, ic, pc);
     GradSum<METHOD, LIM> s;
     s.init(pc, c0);
-    for (int j0 = 0;;) {
+    for (int left = n;;) {
       T pj[CH][4];
 #pragma unroll
       for (int q = 0; q < CH; q++)
-        if (j0 + q < n) ldc4<COH>(P, ch.id[q], pj[q]);
+        if (q < left) ldc4<COH>(P, ch.id[q], pj[q]);
 #pragma unroll
       for (int q = 0; q < CH; q++)
-        if (j0 + q < n) {
+        if (q < left) {
 #if FVS_STRICT
           s.add(pc, pj[q], ch.c[q], ch.w[q]);
 #else
           s.add(pc, pj[q], ch.c[q], T(1));
 #endif
         }
-      j0 += CH;
-      if (j0 >= n) break;
-      ch.load(d, at + 32 * (size_t)j0, n - j0);
+      left -= CH;
+      if (left <= 0) break;
+      ch.load(d, place(ic, n - left), left);
     }
     T ph;
     s.finish(d, ic, pc, ph);
