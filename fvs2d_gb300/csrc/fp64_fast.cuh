@@ -4,7 +4,8 @@
 // GB300 executes 2 FP64 operations per clock per SM, and the FP64 Roe flux
 // is bound by that pipe.  A reciprocal or square root rounded as IEEE
 // division and sqrt require costs several FP64 operations plus special-case
-// handling; the flux needs three reciprocals and two square roots per edge.
+// handling; the flux needs one reciprocal and two reciprocal square roots per
+// edge.
 // Here each starts from PTX's approximate instructions (rcp.approx.ftz.f64,
 // rsqrt.approx.ftz.f64: issued on the special-function unit, not on the FP64
 // pipe) and is refined by ONE Newton-Raphson step carried to second order
@@ -21,10 +22,12 @@
 // over many arguments through fvs_check_fp64_math).  Three FP64 operations
 // for 1/x, five for 1/sqrt x.
 //
-// Domain: positive normal numbers (densities, pressures, squared sound
-// speeds of physical states).  Zero, negative, infinite and NaN arguments
-// give NaN or infinity, which the residual-norm checks report as
-// FVS_ERR_NONFINITE; subnormal arguments are flushed to zero.
+// Domain: normal numbers, for the root positive ones (densities, pressures,
+// squared sound speeds of physical states; the reciprocal takes negative ones
+// too).  Zero, infinite and NaN arguments, and negative ones of the root, give
+// NaN or infinity, which the residual-norm checks report as FVS_ERR_NONFINITE;
+// subnormal arguments are flushed to zero.  A caller that forms a product
+// first (the flux's root of two densities) looks after that product's range.
 #pragma once
 
 namespace fvs {
