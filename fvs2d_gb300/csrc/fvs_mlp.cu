@@ -29,6 +29,7 @@
 #include <cstdint>
 #include <cstring>
 #include <memory>
+#include <new>
 #include <random>
 #include <string>
 #include <vector>
@@ -709,12 +710,18 @@ int fvs_mlp_train(fvs_mlp* m, const float* x, const float* y, int64_t n, int32_t
   if (!m->ensure_rows(batch, true)) return m->fail(FVS_ERR_NOMEM, "activation allocation");
   if (!m->data_x.grow((size_t)n * m->n_in) || !m->data_y.grow((size_t)n * m->n_out) || !m->data_idx.grow((size_t)n))
     return m->fail(FVS_ERR_NOMEM, "dataset allocation");
-  cudaMemcpyAsync(m->data_x.p, x, 4 * (size_t)n * m->n_in, cudaMemcpyHostToDevice, m->stream);
-  cudaMemcpyAsync(m->data_y.p, y, 4 * (size_t)n * m->n_out, cudaMemcpyHostToDevice, m->stream);
   // Orders of the even and of the odd epochs: one is written while the copy of
   // the other may still be in flight (an asynchronous copy from pageable memory
   // may read it after the call has returned); check() ends every epoch.
-  std::vector<int> order[2] = {std::vector<int>(n), std::vector<int>(epochs > 1 ? n : 0)};
+  std::vector<int> order[2];
+  try {
+    order[0].resize((size_t)n);
+    if (epochs > 1) order[1].resize((size_t)n);
+  } catch (const std::bad_alloc&) {
+    return m->fail(FVS_ERR_NOMEM, "sample order");
+  }
+  cudaMemcpyAsync(m->data_x.p, x, 4 * (size_t)n * m->n_in, cudaMemcpyHostToDevice, m->stream);
+  cudaMemcpyAsync(m->data_y.p, y, 4 * (size_t)n * m->n_out, cudaMemcpyHostToDevice, m->stream);
   std::mt19937_64 rng(seed);
   auto shuffle = [&](std::vector<int>& idx) {
     for (int64_t i = 0; i < n; i++) idx[i] = (int)i;
